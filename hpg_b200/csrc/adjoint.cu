@@ -264,6 +264,15 @@ Status linear_op(hpgb_gridder* g, const void* d_vis, size_t n, int op,
                        "too many visibilities for one launch");
   // the tile-sorted kernels (adjoint_tiled.cu) unless the per-visibility
   // kernels are selected or the CF's region does not fit shared memory
+  if (g->kernel_kind == HPGB_KERNEL_AUTO) {
+    bool used = false;
+    HPGB_TRY(linear_op_stream(g, d_vis, n, op, in, out, &used));
+    if (used) {
+      g->last_kernel = linear_tiled_fits(g) ? HPGB_KERNEL_TILED
+                                            : HPGB_KERNEL_DIRECT;
+      return Status::ok();
+    }
+  }
   if (g->kernel_kind != HPGB_KERNEL_DIRECT) {
     bool used = false;
     HPGB_TRY(linear_op_tiled(g, d_vis, n, op, in, out, &used));

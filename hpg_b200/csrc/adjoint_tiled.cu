@@ -331,6 +331,13 @@ __global__ void zero_vals_kernel(double2* v, size_t n) {
 
 }  // namespace
 
+bool linear_tiled_fits(const hpgb_gridder* g) {
+  const int taps = std::max(g->cf.max_taps_x, g->cf.max_taps_y);
+  int R = int(std::sqrt(double(kAdjSmemBudget) / (16.0 * g->grid_size[2])));
+  R = std::min(R, 128) & ~1;
+  return R - taps + 1 >= 4;
+}
+
 // Runs op on the tile sort of the batch; *used is false when the region of
 // the largest CF does not fit shared memory (the caller then uses the
 // per-visibility kernels).

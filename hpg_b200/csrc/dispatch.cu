@@ -1,8 +1,11 @@
 // dispatch.cu -- choice of gridding kernel for one batch.
 //
-// The tiled kernel (grid_tiled.cu) takes every batch whose CF fits its
-// shared-memory ring; the per-visibility kernels (grid_direct.cu) take the
-// rest, or every batch when selected with hpgb_set_gridding_kernel.
+// Automatic: the stream kernel (grid_stream.cu), one visibility per group of
+// warps, takes the batches its plan says it is the faster for; the tiled
+// kernel (grid_tiled.cu) those with large multi-plane CF slices, and every
+// batch when its plan was set by hand or it is selected; the per-visibility
+// kernels (grid_direct.cu) what fits neither, or every batch when selected
+// with hpgb_set_gridding_kernel.
 
 #include "gridder.cuh"
 
@@ -10,6 +13,18 @@ namespace hpgb {
 
 Status grid_batch(hpgb_gridder* g, const void* d_vis, size_t n,
                   unsigned flags) {
+  // the automatic choice, unless the tiled kernel's plan was set by hand
+  if (g->kernel_kind == HPGB_KERNEL_AUTO && g->tplan.ring_parts == 0 &&
+      g->tplan.chunk_vis == 0 && g->tplan.tile_side == 0) {
+    bool used = false;
+    HPGB_TRY(grid_stream(g, const_cast<void*>(d_vis), n, flags, &used));
+    if (used) {
+      int side = 0;
+      g->last_kernel = tiled_plan_side(g, flags, n, &side) ? HPGB_KERNEL_TILED
+                                                           : HPGB_KERNEL_DIRECT;
+      return Status::ok();
+    }
+  }
   if (g->kernel_kind != HPGB_KERNEL_DIRECT) {
     bool used = false;
     HPGB_TRY(grid_tiled(g, const_cast<void*>(d_vis), n, flags, &used));

@@ -23,6 +23,7 @@
 #include <memory>
 #include <vector>
 
+#include "grid_stream.cuh"
 #include "tiled_kernel.cuh"
 
 namespace hpgb {
@@ -69,6 +70,18 @@ __global__ void place_batch_kernel(const __grid_constant__ BatchTable t,
     out[off + k] = c;
   }
   if (j == t.njobs - 1 && threadIdx.x == 0) *total = off + nj;
+}
+
+// the stream kernel's job table, likewise
+struct StreamTable {
+  int njobs;
+  stream::StreamJob jobs[kMaxBatchJobs];
+};
+static_assert(sizeof(StreamTable) <= 32000, "kernel parameter limit");
+
+__global__ void place_stream_jobs_kernel(const __grid_constant__ StreamTable t,
+                                         stream::StreamJob* jobs) {
+  for (int j = threadIdx.x; j < t.njobs; j += blockDim.x) jobs[j] = t.jobs[j];
 }
 
 template <bool MIXED>
@@ -214,6 +227,90 @@ Status grid_batch_launch(hpgb_gridder* const* gs, size_t njobs,
   return launch_batch_n<false>(g0, g0->npol, p, plan.smem, unused);
 }
 
+// The batches of many gridders in one launch of the stream kernel, the
+// gridders' blocks of visibilities one after another over its CTAs; their
+// preparation runs on their own streams.
+Status grid_batch_stream(hpgb_gridder* const* gs, size_t njobs,
+                         void* const* d_vis, const size_t* nvis,
+                         unsigned flags, bool* used) {
+  using namespace stream;
+  *used = false;
+  hpgb_gridder* g0 = gs[0];
+  const bool mixed = g0->precision == HPGB_PRECISION_MIXED;
+  const bool degrid = flags & HPGB_DO_DEGRID, grid = flags & HPGB_DO_GRID;
+  const bool model = degrid && g0->has_model;
+  CFShape cf;
+  size_t total = 0;
+  for (size_t j = 0; j < njobs; ++j) {
+    cf.add(gs[j]);
+    total += nvis[j];
+  }
+  if (total == 0 || njobs > size_t(tiled::kMaxBatchJobs)) return Status::ok();
+  const int(*dset[2])[4] = {g0->mt.m, g0->mt.c};
+  const int(*gset[2])[4] = {g0->mt.c, g0->mt.m};
+  const StreamPlan pl = make_stream_plan(g0, cf, degrid, grid, g0->has_model,
+                                         dset, gset, total, mixed);
+  if (!pl.ok) return Status::ok();
+  *used = true;
+  const cudaStream_t st = g0->stream;
+  cudaEvent_t fork = nullptr;
+  HPGB_CUDA_TRY(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+  std::vector<cudaEvent_t> joins;
+  struct Release {
+    cudaEvent_t& f;
+    std::vector<cudaEvent_t>& j;
+    ~Release() {
+      cudaEventDestroy(f);
+      for (cudaEvent_t e : j) cudaEventDestroy(e);
+    }
+  } release{fork, joins};
+  HPGB_CUDA_TRY(cudaEventRecord(fork, st));
+  std::unique_ptr<StreamTable> table(new StreamTable);
+  std::memset(table.get(), 0, sizeof(StreamTable));
+  for (size_t j = 0; j < njobs; ++j) {
+    hpgb_gridder* g = gs[j];
+    if (nvis[j] == 0) continue;
+    const cudaStream_t js = g->stream;
+    if (js != st) HPGB_CUDA_TRY(cudaStreamWaitEvent(js, fork, 0));
+    StreamPrep prep;
+    HPGB_TRY(prepare_stream(g, d_vis[j], nvis[j],
+                            stream_sorted(g, nvis[j], model), &prep, js));
+    if (model && mixed) HPGB_TRY(tiled::ensure_model32(g, js));
+    StreamJob& b = table->jobs[table->njobs++];
+    b.descs = prep.descs;
+    b.srefs = prep.srefs;
+    b.num_vis = prep.num_vis;
+    b.cf = g->cf.data.as<const float2>();
+    b.model = mixed ? g->model32.ptr : g->model.ptr;
+    b.grid = g->grid.as<double2>();
+    b.weights = g->weights.as<double>();
+    b.records = static_cast<unsigned char*>(d_vis[j]);
+    b.nx = int(g->grid_size[0]);
+    b.ny = int(g->grid_size[1]);
+    if (js != st) {
+      cudaEvent_t e = nullptr;
+      HPGB_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      joins.push_back(e);
+      HPGB_CUDA_TRY(cudaEventRecord(e, js));
+      HPGB_CUDA_TRY(cudaStreamWaitEvent(st, e, 0));
+    }
+  }
+  VisBuffers& vb = g0->vb;
+  HPGB_TRY(vb.batch_jobs.reserve(njobs * std::max(sizeof(BatchJob), sizeof(StreamJob))));
+  place_stream_jobs_kernel<<<1, 128, 0, st>>>(*table,
+                                              vb.batch_jobs.as<StreamJob>());
+  HPGB_CUDA_TRY(cudaGetLastError());
+  ++g0->launches;
+  StreamParams p = pl.p;
+  p.jobs = vb.batch_jobs.as<const StreamJob>();
+  p.njobs = table->njobs;
+  p.update_weights = (flags & HPGB_UPDATE_GRID_WEIGHTS) != 0;
+  p.rec_stride = int(visdata_size(g0->npol));
+  p.status = vb.counters.as<unsigned>();
+  p.wait_limit_ns = g0->wait_limit_ns;
+  return launch_stream(g0, mixed ? stream::kMixed : stream::kFP64, pl, p);
+}
+
 // The gridders are grouped by their widest CF (taps up to 17, 33, 65, more)
 // and by the tile side their own plan would take: one launch's plan -- ring
 // depth and tile side -- is sized for its widest CF and its gridders' tiles
@@ -238,6 +335,16 @@ Status grid_batch_tiled(hpgb_gridder* const* gs, size_t njobs,
                            "gridder " + std::to_string(j) +
                                ": model row pitch not a 16-byte multiple "
                                "(odd grid width in the mixed form)");
+  bool automatic = true;  // the kernel, and the tiled kernel's plan
+  for (size_t j = 0; j < njobs; ++j)
+    automatic = automatic && gs[j]->kernel_kind == HPGB_KERNEL_AUTO &&
+                gs[j]->tplan.ring_parts == 0 && gs[j]->tplan.chunk_vis == 0 &&
+                gs[j]->tplan.tile_side == 0;
+  if (automatic) {
+    bool used = false;
+    HPGB_TRY(grid_batch_stream(gs, njobs, d_vis, nvis, flags, &used));
+    if (used) return Status::ok();
+  }
   auto taps_class = [](const hpgb_gridder* g) {
     const int t = std::max(g->cf.max_taps_x, g->cf.max_taps_y);
     return t <= 17 ? 0 : t <= 33 ? 1 : t <= 65 ? 2 : 3;

@@ -1,0 +1,292 @@
+// grid_stream.cu -- plan of the stream kernel (stream_kernel.cuh) and its
+// launches for one gridder: gridding, degridding and both, and the linear
+// operators.
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "grid_stream.cuh"
+#include "tiled_kernel.cuh"
+
+namespace hpgb {
+namespace stream {
+
+void CFShape::add(const hpgb_gridder* g) {
+  double sum = 0.0;
+  for (const CFGroup& G : g->cf.groups) {
+    max_plane_bytes = std::max(max_plane_bytes, G.plane_stride * 8);
+    max_taps = std::max(max_taps, G.taps_x + G.taps_y);
+    sum += G.plane_stride * 8.0;
+  }
+  if (!g->cf.groups.empty())
+    mean_plane_bytes =
+        std::max(mean_plane_bytes, sum / double(g->cf.groups.size()));
+  table_bytes += g->cf.data.bytes;
+}
+
+// The batch goes into tile order when its footprints cover the grid (and
+// model) several times over and those do not stay in L2 anyway: the sort's
+// ~10 launches and descriptor gathers cost 60-100 us, unsorted footprints in
+// a grid larger than L2 a DRAM read and write of every sector they touch.
+bool stream_sorted(const hpgb_gridder* g, size_t n, bool has_model) {
+  const double grid = 16.0 * double(g->grid_elems()) * (has_model ? 2.0 : 1.0);
+  double cells = 0.0;
+  for (const CFGroup& G : g->cf.groups) cells += double(G.taps_x) * G.taps_y;
+  cells /= std::max<size_t>(g->cf.groups.size(), 1);
+  const double touched =
+      double(n) * cells * double(g->grid_size[2]) * 16.0;
+  return grid > 64e6 && touched > 2.0 * grid;
+}
+
+StreamPlan make_stream_plan(const hpgb_gridder* g, const CFShape& cf,
+                            bool degrid, bool grid, bool has_model,
+                            const int (*const dset[2])[4],
+                            const int (*const gset[2])[4], size_t nvis,
+                            bool tiles_fp32) {
+  StreamPlan pl;
+  StreamParams& p = pl.p;
+  std::memset(&p, 0, sizeof(p));
+  const int nrow = int(g->grid_size[2]), n = int(g->npol);
+  if (nrow < 1 || nrow > 4 || g->cf.groups.empty()) return pl;
+  p.nrow = nrow;
+  p.ncube = int(g->grid_size[3]);
+  p.do_degrid = degrid;
+  p.do_grid = grid;
+  p.has_model = has_model;
+  const bool use_d = degrid && has_model, use_g = grid;
+  // one active element per row, the same for both signs of w, and a row per
+  // polarization
+  pl.diag = nrow == n;
+  for (int r = 0; r < nrow && pl.diag; ++r) {
+    int act[4] = {0, 0, 0, 0}, cnt = 0;
+    for (int v = 0; v < n; ++v) {
+      int on = 0, all = 0;
+      for (int w = 0; w < 2; ++w) {
+        if (use_d) on += dset[w][r][v] >= 0, ++all;
+        if (use_g) on += gset[w][r][v] >= 0, ++all;
+      }
+      if (on != 0 && on != all) pl.diag = false;
+      act[v] = on != 0;
+      cnt += act[v];
+      if (act[v]) p.vact[r] = v;
+    }
+    pl.diag = pl.diag && cnt == 1;
+  }
+  if (n == 1 && !pl.diag) return pl;
+  // planes used, and their places: in a ring slot, or in the slice
+  bool need[64] = {false};
+  for (int r = 0; r < nrow; ++r)
+    for (int v = 0; v < n; ++v)
+      for (int w = 0; w < 2; ++w)
+        for (int set = 0; set < 2; ++set) {
+          if (!(set ? use_g : use_d)) continue;
+          const int m = (set ? gset : dset)[w][r][v];
+          if (m >= 64) return pl;
+          if (m >= 0) need[m] = true;
+        }
+  int pos[64], np = 0, nr = 0;
+  bool runs_fit = true;
+  for (int m = 0; m < 64; ++m) {
+    pos[m] = -1;
+    if (!need[m]) continue;
+    pos[m] = np;
+    if (m > 0 && need[m - 1]) {
+      if (runs_fit) p.run_len[nr - 1]++;
+    } else if (nr == kMaxRuns) {
+      runs_fit = false;
+    } else {
+      p.run_plane[nr] = m;
+      p.run_len[nr] = 1;
+      p.run_dst[nr] = np;
+      ++nr;
+    }
+    ++np;
+  }
+  p.nplanes = np;
+  p.nruns = nr;
+  // shared memory: partial sums and screen tables per group, then the ring
+  const int kBudget = 227 * 1024;
+  const int part = (np * cf.max_plane_bytes + 127) / 128 * 128;
+  const double mean = np * cf.mean_plane_bytes;
+  p.tab_taps = cf.max_taps;
+  auto layout = [&](int warps, bool ring) {
+    const int groups = (ring ? kWarps - kProducers : kFreeWarps) / warps;
+    p.off_part = ring ? Fixed::kEnd : 0;
+    p.off_offs = (p.off_part + groups * warps * 2 * n * 8 + 15) / 16 * 16;
+    p.off_tab = p.off_offs + kWarps * 32 * 4;
+    p.off_ring = (p.off_tab + groups * p.tab_taps * 16 + 127) / 128 * 128;
+    return p.off_ring;
+  };
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device);
+  const double cells = cf.mean_plane_bytes / 8.0;
+  if (pl.diag) {
+    // One plane per row: read from global memory (a bulk copy each, ~430
+    // cycles per SM whatever its size, bounds the kernel: supports 8 to 32,
+    // one polarization, 1M visibilities degridded 1.6 against 3.7 ms), a
+    // warp per visibility, two when footprints are wide (2 polarizations,
+    // supports 8 to 64, 500k visibilities, both passes: 8.4 against 8.8 ms;
+    // degridding 2.8 against 2.5), four when there are too few visibilities
+    // for every warp.
+    pl.warps = cells < 128 || nvis >= size_t(sms) * 32 ? (cells > 1024 ? 2 : 1) : 4;
+    // FP32 grid tiles take a wide footprint's additions faster than the
+    // grid's FP64 reductions do (that configuration, gridding only: 5.0
+    // against 6.8 ms; the FP64 form's tiles do not, 8.0 against 6.8).
+    if (tiles_fp32 && !use_d && cells > 900) return pl;
+  } else {
+    // Several planes per row: through the ring from 10 KB of slice on (4x4
+    // planes, supports 8 to 16, 300k visibilities, both passes: 2.7 against
+    // 5.4 ms; below, supports 4 to 8, 1M: 5.3 against 4.7 ms, but degridding
+    // 3.1 against 3.9, gridding 3.4 against 4.3).  Beyond 48 KB the ring
+    // holds too few visibilities, and the tiled kernel, which splits a slice
+    // over the CTAs of a cluster, is faster (supports 8 to 32: 183 ms
+    // per 10M visibilities against 315) once its pipeline has work: 5k
+    // visibilities take 0.63 ms there, 0.49 here.
+    pl.ring = mean >= 10 * 1024;
+    if (pl.ring && part > 48 * 1024 && nvis > 5000) return pl;
+    pl.warps = !pl.ring ? 1 : part > 40 * 1024 ? 7 : 2;
+    if (pl.ring && !(runs_fit && np > 0 &&
+                     layout(pl.warps, true) + part <= kBudget - 1024))
+      return pl;
+  }
+  if (pl.ring) {
+    layout(pl.warps, true);
+    p.ring_bytes = (kBudget - 1024 - p.off_ring) / 1024 * 1024;
+    pl.smem = p.off_ring + p.ring_bytes;
+  } else {
+    pl.smem = std::max(layout(pl.warps, false), 1024);
+    if (pl.smem * ctas_per_sm(false, n) > kBudget) return pl;
+  }
+  for (int r = 0; r < nrow; ++r)
+    for (int w = 0; w < 2; ++w)
+      for (int k = 0; k < (pl.diag ? 1 : n); ++k) {
+        const int v = pl.diag ? p.vact[r] : k;
+        auto place = [&](int m) {
+          return uint32_t((m < 0 ? -1 : pl.ring ? pos[m] : m) & 0xff);
+        };
+        if (use_d) p.dpack[r][w] |= place(dset[w][r][v]) << (8 * k);
+        if (use_g) p.gpack[r][w] |= place(gset[w][r][v]) << (8 * k);
+      }
+  // every element of every row active
+  p.dense = 1;
+  for (int r = 0; r < nrow; ++r)
+    for (int w = 0; w < 2; ++w)
+      for (int v = 0; v < n; ++v) {
+        if (use_d && dset[w][r][v] < 0) p.dense = 0;
+        if (use_g && gset[w][r][v] < 0) p.dense = 0;
+      }
+  p.evict_first = cf.table_bytes > size_t(96) << 20;
+  pl.ctas = sms * ctas_per_sm(pl.ring, n);
+  p.block_vis = int(std::min<size_t>(
+      kBlockVis, std::max<size_t>(1, (nvis + pl.ctas - 1) / size_t(pl.ctas))));
+  pl.ok = true;
+  return pl;
+}
+
+Status launch_stream(hpgb_gridder* g, int form, const StreamPlan& pl,
+                     const StreamParams& p) {
+  auto with = [&](auto f) -> Status {
+    constexpr int F = decltype(f)::value;
+    switch (g->npol) {
+      case 1: return launch_stream_n<F, 1>(g, pl, p);
+      case 2: return launch_stream_n<F, 2>(g, pl, p);
+      case 3: return launch_stream_n<F, 3>(g, pl, p);
+      case 4: return launch_stream_n<F, 4>(g, pl, p);
+      default: return Status::err(HPGB_ERROR_OTHER, "bad polarization count");
+    }
+  };
+  if (form == kLinear) return with(std::integral_constant<int, kLinear>());
+  if (form == kMixed) return with(std::integral_constant<int, kMixed>());
+  return with(std::integral_constant<int, kFP64>());
+}
+
+}  // namespace stream
+
+using namespace stream;
+
+Status grid_stream(hpgb_gridder* g, void* d_vis, size_t n, unsigned flags,
+                   bool* used) {
+  *used = false;
+  const bool degrid = flags & HPGB_DO_DEGRID, grid = flags & HPGB_DO_GRID;
+  if (n == 0 || n > size_t(0x7fffffff) || !(degrid || grid))
+    return Status::ok();
+  const bool mixed = g->precision == HPGB_PRECISION_MIXED;
+  // (the mixed form degrids odd grid widths in FP64, by the kernels that do
+  // not need its FP32 model)
+  if (mixed && degrid && g->has_model && (g->grid_size[0] & 1))
+    return Status::ok();
+  // pos_w (w = 1): degrid uses conjugate indexes, grid uses indexes
+  const int(*dset[2])[4] = {g->mt.m, g->mt.c};
+  const int(*gset[2])[4] = {g->mt.c, g->mt.m};
+  CFShape cf;
+  cf.add(g);
+  const StreamPlan pl = make_stream_plan(g, cf, degrid, grid, g->has_model,
+                                         dset, gset, n, mixed);
+  if (!pl.ok) return Status::ok();
+  *used = true;
+  StreamPrep prep;
+  HPGB_TRY(prepare_stream(g, d_vis, n,
+                          stream_sorted(g, n, degrid && g->has_model), &prep,
+                          g->stream));
+  if (mixed && degrid && g->has_model)
+    HPGB_TRY(tiled::ensure_model32(g, g->stream));
+  StreamParams p = pl.p;
+  p.job.descs = prep.descs;
+  p.job.srefs = prep.srefs;
+  p.job.num_vis = prep.num_vis;
+  p.job.cf = g->cf.data.as<const float2>();
+  p.job.model = mixed ? g->model32.ptr : g->model.ptr;
+  p.job.grid = g->grid.as<double2>();
+  p.job.weights = g->weights.as<double>();
+  p.job.records = static_cast<unsigned char*>(d_vis);
+  p.job.nx = int(g->grid_size[0]);
+  p.job.ny = int(g->grid_size[1]);
+  p.update_weights = (flags & HPGB_UPDATE_GRID_WEIGHTS) != 0;
+  p.rec_stride = int(visdata_size(g->npol));
+  p.status = g->vb.counters.as<unsigned>();
+  p.wait_limit_ns = g->wait_limit_ns;
+  return launch_stream(g, mixed ? kMixed : kFP64, pl, p);
+}
+
+Status linear_op_stream(hpgb_gridder* g, const void* d_vis, size_t n, int op,
+                        const void* in, void* out, bool* used) {
+  *used = false;
+  if (n == 0 || n > size_t(0x7fffffff)) return Status::ok();
+  const bool gather = op == 0 || op == 3;
+  // D and D^H use the degridding indexes, G and G^H the gridding ones
+  const int(*set[2])[4] = {g->mt.m, g->mt.c};
+  if (op >= 2) std::swap(set[0], set[1]);
+  CFShape cf;
+  cf.add(g);
+  const StreamPlan pl =
+      make_stream_plan(g, cf, gather, !gather, gather, set, set, n, false);
+  if (!pl.ok) return Status::ok();
+  *used = true;
+  StreamPrep prep;
+  HPGB_TRY(prepare_stream(g, const_cast<void*>(d_vis), n,
+                          stream_sorted(g, n, false), &prep, g->stream));
+  StreamParams p = pl.p;
+  p.op = op;
+  p.job.descs = prep.descs;
+  p.job.srefs = prep.srefs;
+  p.job.num_vis = prep.num_vis;
+  p.job.cf = g->cf.data.as<const float2>();
+  p.job.nx = int(g->grid_size[0]);
+  p.job.ny = int(g->grid_size[1]);
+  if (gather) {
+    p.job.model = in;
+    p.vals_out = static_cast<double2*>(out);
+    // visibilities off the grid get zero
+    HPGB_CUDA_TRY(cudaMemsetAsync(out, 0, n * g->npol * sizeof(double2),
+                                  g->stream));
+  } else {
+    p.vals_in = static_cast<const double2*>(in);
+    p.job.grid = static_cast<double2*>(out);
+  }
+  p.status = g->vb.counters.as<unsigned>();
+  p.wait_limit_ns = g->wait_limit_ns;
+  return launch_stream(g, kLinear, pl, p);
+}
+
+}  // namespace hpgb

@@ -146,33 +146,19 @@ __global__ void chunk_write_kernel(const unsigned* counts,
   if (t == ntiles - 1) *num_chunks = cstart[t] + nch[t];
 }
 
+// the descriptor and slice reference of visibility i (on the grid at vc), its
+// footprint origin relative to (x0, y0)
 template <int N>
-__global__ void tile_desc_kernel(const VisData<N>* vis, const unsigned* order,
-                                 const unsigned* keys, size_t n, GridGeom g,
-                                 const CFGroup* groups, TileGeom tg,
-                                 const float2* cf_base, TileDesc* descs,
-                                 SliceRef* srefs, const unsigned* tstart,
-                                 const unsigned* tcount) {
-  const size_t pidx = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-  if (pidx >= n) return;
-  const unsigned key = keys[pidx] >> tg.sbits;  // the tile
-  if (key >= unsigned(tg.ntiles)) return;
-  // the tile's visibilities are sorted by footprint size; descriptor
-  // position pidx takes the one tile_order_source picks
-  const unsigned t0 = tstart[key];
-  const unsigned r = unsigned(pidx) - t0;
-  const unsigned i = order[t0 + tile_order_source(r, tcount[key], tg.order)];
-  const VisData<N>& vd = vis[i];
-  VisCoord vc;
-  vis_coords(g, groups, vd.freq, vd.uvw, vd.grid_cube, vd.cf_index,
-             vd.cf_phase_gradient, vc);
+__device__ __forceinline__ void make_desc(const VisData<N>& vd, unsigned i,
+                                          const VisCoord& vc, int x0, int y0,
+                                          const GridGeom& g,
+                                          const CFGroup* groups,
+                                          const float2* cf_base, TileDesc& d,
+                                          SliceRef& s) {
   const CFGroup& G = groups[vc.grp];
-  const int tx = int(key % unsigned(tg.ntx));
-  const int ty = int((key / unsigned(tg.ntx)) % unsigned(tg.nty));
-  TileDesc d;
   d.index = int(i);
-  d.cx = int16_t(vc.grid_coord[0] - tx * tg.T);
-  d.cy = int16_t(vc.grid_coord[1] - ty * tg.T);
+  d.cx = int16_t(vc.grid_coord[0] - x0);
+  d.cy = int16_t(vc.grid_coord[1] - y0);
   d.taps_x = uint8_t(vc.taps[0]);
   d.taps_y = uint8_t(vc.taps[1]);
   const bool screen_on = vc.phi0[0] != 0.0 || vc.phi0[1] != 0.0 ||
@@ -225,12 +211,97 @@ __global__ void tile_desc_kernel(const VisData<N>* vis, const unsigned* order,
     d.twgt[r] = tw;
   }
   d.inv_tx = 1.0f / float(vc.taps[0]);
-  for (int k = 0; k < 3; ++k) d.pad1[k] = 0;
-  descs[pidx] = d;
-  SliceRef s;
+  d.abs_x = vc.grid_coord[0];
+  d.abs_y = vc.grid_coord[1];
+  d.cube = vc.grid_cube;
   s.off = (G.data - cf_base) + sidx * G.slice_stride;
   s.pstride = G.plane_stride;
   s.ncell = vc.taps[0] * vc.taps[1];
+}
+
+template <int N>
+__global__ void tile_desc_kernel(const VisData<N>* vis, const unsigned* order,
+                                 const unsigned* keys, size_t n, GridGeom g,
+                                 const CFGroup* groups, TileGeom tg,
+                                 const float2* cf_base, TileDesc* descs,
+                                 SliceRef* srefs, const unsigned* tstart,
+                                 const unsigned* tcount) {
+  const size_t pidx = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+  if (pidx >= n) return;
+  const unsigned key = keys[pidx] >> tg.sbits;  // the tile
+  if (key >= unsigned(tg.ntiles)) return;
+  // the tile's visibilities are sorted by footprint size; descriptor
+  // position pidx takes the one tile_order_source picks
+  const unsigned t0 = tstart[key];
+  const unsigned r = unsigned(pidx) - t0;
+  const unsigned i = order[t0 + tile_order_source(r, tcount[key], tg.order)];
+  const VisData<N>& vd = vis[i];
+  VisCoord vc;
+  vis_coords(g, groups, vd.freq, vd.uvw, vd.grid_cube, vd.cf_index,
+             vd.cf_phase_gradient, vc);
+  const int tx = int(key % unsigned(tg.ntx));
+  const int ty = int((key / unsigned(tg.ntx)) % unsigned(tg.nty));
+  TileDesc d;
+  SliceRef s;
+  make_desc<N>(vd, i, vc, tx * tg.T, ty * tg.T, g, groups, cf_base, d, s);
+  descs[pidx] = d;
+  srefs[pidx] = s;
+}
+
+// keys of the tile order without passes, and the number of visibilities on
+// the grid
+template <int N>
+__global__ void stream_keys_kernel(const VisData<N>* vis, size_t n, GridGeom g,
+                                   const CFGroup* groups, int ntx, int nty,
+                                   unsigned* keys, unsigned* order,
+                                   unsigned* num_vis) {
+  const size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+  bool on = false;
+  if (i < n) {
+    const VisData<N>& vd = vis[i];
+    VisCoord vc;
+    vis_coords(g, groups, vd.freq, vd.uvw, vd.grid_cube, vd.cf_index,
+               vd.cf_phase_gradient, vc);
+    on = vc.in_grid;
+    keys[i] = on ? unsigned((vc.grid_cube * nty +
+                             vc.grid_coord[1] / kStreamTile) * ntx +
+                            vc.grid_coord[0] / kStreamTile)
+                 : unsigned(g.ncube * nty * ntx);
+    order[i] = unsigned(i);
+  }
+  const int count = __syncthreads_count(on);
+  if (threadIdx.x == 0 && count > 0) atomicAdd(num_vis, unsigned(count));
+}
+
+// order: the sorted order (num_vis of them on the grid), or null: as in the
+// batch, those off the grid flagged
+template <int N>
+__global__ void stream_desc_kernel(const VisData<N>* vis, const unsigned* order,
+                                   size_t n, GridGeom g, const CFGroup* groups,
+                                   const float2* cf_base, TileDesc* descs,
+                                   SliceRef* srefs, unsigned* num_vis) {
+  const size_t pidx = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+  if (!order && pidx == 0) *num_vis = unsigned(n);
+  if (pidx >= (order ? size_t(*num_vis) : n)) return;
+  const unsigned i = order ? order[pidx] : unsigned(pidx);
+  const VisData<N>& vd = vis[i];
+  VisCoord vc;
+  vis_coords(g, groups, vd.freq, vd.uvw, vd.grid_cube, vd.cf_index,
+             vd.cf_phase_gradient, vc);
+  TileDesc d;
+  SliceRef s;
+  if (vc.in_grid) {
+    make_desc<N>(vd, i, vc, vc.grid_coord[0], vc.grid_coord[1], g, groups,
+                 cf_base, d, s);
+    descs[pidx] = d;
+  } else {
+    // (a slice of one 16-byte unit per plane, never used)
+    descs[pidx].taps_x = descs[pidx].taps_y = 0;
+    descs[pidx].flags = kSkip;
+    s.off = 0;
+    s.pstride = 2;
+    s.ncell = 0;
+  }
   srefs[pidx] = s;
 }
 
@@ -264,6 +335,18 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
+Status ensure_model32(hpgb_gridder* g, cudaStream_t st) {
+  if (g->model32_valid) return Status::ok();
+  const size_t ne = g->grid_elems();
+  HPGB_TRY(g->model32.reserve(std::max<size_t>(ne, 1) * sizeof(float2)));
+  model_to_f32_kernel<<<148 * 8, 256, 0, st>>>(
+      g->model.as<const double2>(), g->model32.as<float2>(), ne);
+  HPGB_CUDA_TRY(cudaGetLastError());
+  ++g->launches;
+  g->model32_valid = true;
+  return Status::ok();
+}
+
 Status encode_model_map(hpgb_gridder* g, bool mixed, int R, CUtensorMap* map,
                         cudaStream_t st) {
   std::memset(map, 0, sizeof(*map));
@@ -273,15 +356,7 @@ Status encode_model_map(hpgb_gridder* g, bool mixed, int R, CUtensorMap* map,
   size_t esize = 8;
   CUtensorMapDataType dt = CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
   if (mixed) {
-    const size_t ne = g->grid_elems();
-    if (!g->model32_valid) {
-      HPGB_TRY(g->model32.reserve(std::max<size_t>(ne, 1) * sizeof(float2)));
-      model_to_f32_kernel<<<148 * 8, 256, 0, st>>>(
-          g->model.as<const double2>(), g->model32.as<float2>(), ne);
-      HPGB_CUDA_TRY(cudaGetLastError());
-      ++g->launches;
-      g->model32_valid = true;
-    }
+    HPGB_TRY(ensure_model32(g, st));
     base = g->model32.ptr;
     esize = 4;
     dt = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
@@ -622,6 +697,70 @@ Status grid_tiled_n(hpgb_gridder* g, void* d_vis, size_t n, unsigned flags,
 }
 
 }  // namespace
+
+namespace {
+
+template <int N>
+Status prepare_stream_n(hpgb_gridder* g, void* d_vis, size_t n, bool sorted,
+                        StreamPrep* out, cudaStream_t st) {
+  VisBuffers& vb = g->vb;
+  const GridGeom geom = g->geom();
+  const CFGroup* groups = g->cf.desc.as<const CFGroup>();
+  const VisData<N>* vis = static_cast<const VisData<N>*>(d_vis);
+  const unsigned blocks = unsigned((n + 255) / 256);
+  HPGB_TRY(vb.prep.reserve(n * (sizeof(TileDesc) + sizeof(SliceRef))));
+  TileDesc* descs = vb.prep.as<TileDesc>();
+  SliceRef* srefs = reinterpret_cast<SliceRef*>(vb.prep.as<char>() +
+                                                n * sizeof(TileDesc));
+  unsigned* num_vis = vb.counters.as<unsigned>() + 5;
+  const unsigned* order = nullptr;
+  if (sorted) {
+    const int ntx = (geom.nx + kStreamTile - 1) / kStreamTile;
+    const int nty = (geom.ny + kStreamTile - 1) / kStreamTile;
+    HPGB_TRY(vb.keys.reserve(n * 4));
+    HPGB_TRY(vb.keys_alt.reserve(n * 4));
+    HPGB_TRY(vb.order.reserve(n * 4));
+    HPGB_TRY(vb.order_alt.reserve(n * 4));
+    int end_bit = 1;
+    while ((1ll << end_bit) <= (long long)ntx * nty * geom.ncube) ++end_bit;
+    cub::DoubleBuffer<unsigned> kbuf(vb.keys.as<unsigned>(), vb.keys_alt.as<unsigned>());
+    cub::DoubleBuffer<unsigned> vbuf(vb.order.as<unsigned>(), vb.order_alt.as<unsigned>());
+    size_t bytes = 0;
+    HPGB_CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, bytes, kbuf, vbuf,
+                                                  int(n), 0, end_bit, st));
+    HPGB_TRY(vb.sort_tmp.reserve(bytes + 16));
+    HPGB_CUDA_TRY(cudaMemsetAsync(num_vis, 0, sizeof(unsigned), st));
+    stream_keys_kernel<N><<<blocks, 256, 0, st>>>(
+        vis, n, geom, groups, ntx, nty, vb.keys.as<unsigned>(),
+        vb.order.as<unsigned>(), num_vis);
+    HPGB_CUDA_TRY(cudaGetLastError());
+    ++g->launches;
+    bytes = vb.sort_tmp.bytes;
+    HPGB_CUDA_TRY(cub::DeviceRadixSort::SortPairs(vb.sort_tmp.ptr, bytes, kbuf,
+                                                  vbuf, int(n), 0, end_bit, st));
+    order = vbuf.Current();
+  }
+  stream_desc_kernel<N><<<blocks, 256, 0, st>>>(
+      vis, order, n, geom, groups, g->cf.data.as<const float2>(), descs, srefs,
+      num_vis);
+  HPGB_CUDA_TRY(cudaGetLastError());
+  ++g->launches;
+  *out = StreamPrep{descs, srefs, num_vis};
+  return Status::ok();
+}
+
+}  // namespace
+
+Status prepare_stream(hpgb_gridder* g, void* d_vis, size_t n, bool sorted,
+                      StreamPrep* out, cudaStream_t st) {
+  switch (g->npol) {
+    case 1: return prepare_stream_n<1>(g, d_vis, n, sorted, out, st);
+    case 2: return prepare_stream_n<2>(g, d_vis, n, sorted, out, st);
+    case 3: return prepare_stream_n<3>(g, d_vis, n, sorted, out, st);
+    case 4: return prepare_stream_n<4>(g, d_vis, n, sorted, out, st);
+    default: return Status::err(HPGB_ERROR_OTHER, "bad polarization count");
+  }
+}
 
 Status prepare_tiles(hpgb_gridder* g, void* d_vis, size_t n, int T, int ntx,
                      int nty, int K, TilePrep* out, cudaStream_t st,

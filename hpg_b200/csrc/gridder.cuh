@@ -140,6 +140,11 @@ Status copy_cf(hpgb_gridder* dst, const hpgb_gridder* src);
 Status grid_tiled(hpgb_gridder* g, void* d_vis, size_t n, unsigned flags,
                   bool* used);
 
+// grid_stream.cu: one visibility per group of warps, straight into the grid;
+// *used is false when it cannot take the batch
+Status grid_stream(hpgb_gridder* g, void* d_vis, size_t n, unsigned flags,
+                   bool* used);
+
 // grid_tiled.cu: the uv tile side of the plan the tiled kernel would take
 // for the batch (false when no plan fits)
 bool tiled_plan_side(const hpgb_gridder* g, unsigned flags, size_t n,
@@ -176,6 +181,12 @@ Status linear_op(hpgb_gridder* g, const void* d_vis, size_t n, int op,
 // when the CF's tile region does not fit shared memory
 Status linear_op_tiled(hpgb_gridder* g, const void* d_vis, size_t n, int op,
                        const void* in, void* out, bool* used);
+
+bool linear_tiled_fits(const hpgb_gridder* g);
+// grid_stream.cu: the same, one visibility per group of warps; *used is false
+// when it cannot take the batch
+Status linear_op_stream(hpgb_gridder* g, const void* d_vis, size_t n, int op,
+                        const void* in, void* out, bool* used);
 
 // imaging.cu
 Status normalize_by_weights(hpgb_gridder* g, double wfactor);

@@ -222,6 +222,17 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src,
       : "memory");
 }
 
+// the same with an L2 eviction policy (createpolicy) for the source's lines
+__device__ __forceinline__ void bulk_g2s_hint(void* dst, const void* src,
+                                              uint32_t bytes, uint64_t* bar,
+                                              uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::"
+      "cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(smem(dst)),
+      "l"(src), "r"(bytes), "r"(smem(bar)), "l"(policy)
+      : "memory");
+}
+
 // 3-D tiled tensor load (no multicast); c0 is the innermost coordinate
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map,
                                             int c0, int c1, int c2,

@@ -1118,6 +1118,9 @@ struct Plan {
 Plan make_plan(const hpgb_gridder* g, unsigned flags, bool mixed, size_t nvis,
                const BatchShape* batch);
 
+// the FP32 copy of g's model for the mixed form, made on st when missing
+Status ensure_model32(hpgb_gridder* g, cudaStream_t st);
+
 // the 3-D tensor map of g's model (FP32 copy made on st when mixed) with a
 // box of R x R cells of one grid row
 Status encode_model_map(hpgb_gridder* g, bool mixed, int R, CUtensorMap* map,

@@ -27,11 +27,11 @@ struct alignas(16) TileDesc {
   double twgt[4];        // grid weight increment per grid row
   float2 gvis[4];        // values scaled for gridding (used without degrid)
   float inv_tx;          // 1 / taps_x, rounded to float
-  int32_t pad1[3];
+  int32_t abs_x, abs_y, cube;  // footprint origin in the grid
 };
 static_assert(sizeof(TileDesc) == 256, "TileDesc is one 256-byte bulk copy");
 
-enum : uint8_t { kPosW = 1, kScreen = 2 };
+enum : uint8_t { kPosW = 1, kScreen = 2, kSkip = 4 };  // kSkip: off the grid
 
 struct SliceRef {
   long long off;  // float2 offset of the slice in the CF region
@@ -100,5 +100,19 @@ struct TilePrep {
 Status prepare_tiles(hpgb_gridder* g, void* d_vis, size_t n, int T, int ntx,
                      int nty, int K, TilePrep* out, cudaStream_t st = nullptr,
                      int order = kOrderPairs);
+
+// The same without passes, for the kernels that take visibilities one by one
+// (stream_kernel.cuh): descriptors and slice references in the order of uv
+// tiles of kStreamTile cells, or as in the batch (visibilities off the grid
+// flagged kSkip) when sorted is false.  num_vis: device word, the descriptors
+// to take.
+constexpr int kStreamTile = 64;
+struct StreamPrep {
+  const TileDesc* descs;
+  const SliceRef* srefs;
+  const unsigned* num_vis;
+};
+Status prepare_stream(hpgb_gridder* g, void* d_vis, size_t n, bool sorted,
+                      StreamPrep* out, cudaStream_t st);
 
 }  // namespace hpgb

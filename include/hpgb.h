@@ -441,7 +441,9 @@ HPGB_API int hpgb_debug_withhold_copy(hpgb_gridder* gridder,
 /* Which kernel gridded/degridded the gridder's last non-empty batch:
  * HPGB_KERNEL_TILED or HPGB_KERNEL_DIRECT (HPGB_KERNEL_AUTO before the first
  * batch).  No counterpart in the reference: it makes the tiled kernel's
- * fallback to the per-visibility kernels visible to the caller. */
+ * fallback to the per-visibility kernels visible to the caller.  The
+ * automatic choice's own kernel (one visibility per group of warps) counts as
+ * TILED where the tiled kernel could have taken the batch, else as DIRECT. */
 HPGB_API int hpgb_last_gridding_kernel(const hpgb_gridder* gridder,
                                        int* kind);
 
