@@ -17,6 +17,7 @@ void CFShape::add(const hpgb_gridder* g) {
   for (const CFGroup& G : g->cf.groups) {
     max_plane_bytes = std::max(max_plane_bytes, G.plane_stride * 8);
     max_taps = std::max(max_taps, G.taps_x + G.taps_y);
+    max_side = std::max(max_side, std::max(G.taps_x, G.taps_y));
     sum += G.plane_stride * 8.0;
   }
   if (!g->cf.groups.empty())
@@ -48,7 +49,9 @@ StreamPlan make_stream_plan(const hpgb_gridder* g, const CFShape& cf,
   StreamParams& p = pl.p;
   std::memset(&p, 0, sizeof(p));
   const int nrow = int(g->grid_size[2]), n = int(g->npol);
-  if (nrow < 1 || nrow > 4 || g->cf.groups.empty()) return pl;
+  // (the cell loops' row arithmetic holds for supports below 128)
+  if (nrow < 1 || nrow > 4 || g->cf.groups.empty() || cf.max_side > 127)
+    return pl;
   p.nrow = nrow;
   p.ncube = int(g->grid_size[3]);
   p.do_degrid = degrid;

@@ -20,6 +20,7 @@ struct StreamPlan {
 struct CFShape {
   int max_plane_bytes = 0;  // largest plane
   int max_taps = 0;         // taps_x + taps_y, largest
+  int max_side = 0;         // widest footprint
   double mean_plane_bytes = 0;  // over the groups
   size_t table_bytes = 0;
   void add(const hpgb_gridder* g);
