@@ -249,7 +249,7 @@ Status grid_batch_stream(hpgb_gridder* const* gs, size_t njobs,
   const int(*dset[2])[4] = {g0->mt.m, g0->mt.c};
   const int(*gset[2])[4] = {g0->mt.c, g0->mt.m};
   const StreamPlan pl = make_stream_plan(g0, cf, degrid, grid, g0->has_model,
-                                         dset, gset, total, mixed);
+                                         dset, gset, total, mixed, true);
   if (!pl.ok) return Status::ok();
   *used = true;
   const cudaStream_t st = g0->stream;

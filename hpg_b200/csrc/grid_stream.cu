@@ -44,7 +44,7 @@ StreamPlan make_stream_plan(const hpgb_gridder* g, const CFShape& cf,
                             bool degrid, bool grid, bool has_model,
                             const int (*const dset[2])[4],
                             const int (*const gset[2])[4], size_t nvis,
-                            bool tiles_fp32) {
+                            bool tiles_fp32, bool tiled_takes) {
   StreamPlan pl;
   StreamParams& p = pl.p;
   std::memset(&p, 0, sizeof(p));
@@ -114,7 +114,8 @@ StreamPlan make_stream_plan(const hpgb_gridder* g, const CFShape& cf,
   const double mean = np * cf.mean_plane_bytes;
   p.tab_taps = cf.max_taps;
   auto layout = [&](int warps, bool ring) {
-    const int groups = (ring ? kWarps - kProducers : kFreeWarps) / warps;
+    const int groups =
+        (ring ? kWarps - kProducers : warps_of(false, warps)) / warps;
     p.off_part = ring ? Fixed::kEnd : 0;
     p.off_offs = (p.off_part + groups * warps * 2 * n * 8 + 15) / 16 * 16;
     p.off_tab = p.off_offs + kWarps * 32 * 4;
@@ -147,11 +148,20 @@ StreamPlan make_stream_plan(const hpgb_gridder* g, const CFShape& cf,
     // per 10M visibilities against 315) once its pipeline has work: 5k
     // visibilities take 0.63 ms there, 0.49 here.
     pl.ring = mean >= 10 * 1024;
-    if (pl.ring && part > 48 * 1024 && nvis > 5000) return pl;
     pl.warps = !pl.ring ? 1 : part > 40 * 1024 ? 7 : 2;
     if (pl.ring && !(runs_fit && np > 0 &&
-                     layout(pl.warps, true) + part <= kBudget - 1024))
+                     layout(pl.warps, true) + part <= kBudget - 1024)) {
+      // Slices beyond the ring and the tiled kernel (4x4 planes of supports
+      // beyond 45) go to groups of 16 warps, one visibility per SM, whose
+      // slices, read again for gridding, stay in L2 (supports 48 and 64, 20k
+      // visibilities: 7.0 ms; groups of 8, two per SM, 7.9; the
+      // per-visibility kernels 8.7).
+      if (tiled_takes) return pl;
+      pl.ring = false;
+      pl.warps = 16;
+    } else if (pl.ring && part > 48 * 1024 && nvis > 4000) {
       return pl;
+    }
   }
   if (pl.ring) {
     layout(pl.warps, true);
@@ -159,7 +169,7 @@ StreamPlan make_stream_plan(const hpgb_gridder* g, const CFShape& cf,
     pl.smem = p.off_ring + p.ring_bytes;
   } else {
     pl.smem = std::max(layout(pl.warps, false), 1024);
-    if (pl.smem * ctas_per_sm(false, n) > kBudget) return pl;
+    if (pl.smem * ctas_per_sm(false, n, pl.warps) > kBudget) return pl;
   }
   for (int r = 0; r < nrow; ++r)
     for (int w = 0; w < 2; ++w)
@@ -180,7 +190,7 @@ StreamPlan make_stream_plan(const hpgb_gridder* g, const CFShape& cf,
         if (use_g && gset[w][r][v] < 0) p.dense = 0;
       }
   p.evict_first = cf.table_bytes > size_t(96) << 20;
-  pl.ctas = sms * ctas_per_sm(pl.ring, n);
+  pl.ctas = sms * ctas_per_sm(pl.ring, n, pl.warps);
   p.block_vis = int(std::min<size_t>(
       kBlockVis, std::max<size_t>(1, (nvis + pl.ctas - 1) / size_t(pl.ctas))));
   pl.ok = true;
@@ -224,8 +234,10 @@ Status grid_stream(hpgb_gridder* g, void* d_vis, size_t n, unsigned flags,
   const int(*gset[2])[4] = {g->mt.c, g->mt.m};
   CFShape cf;
   cf.add(g);
-  const StreamPlan pl = make_stream_plan(g, cf, degrid, grid, g->has_model,
-                                         dset, gset, n, mixed);
+  int side = 0;
+  const StreamPlan pl =
+      make_stream_plan(g, cf, degrid, grid, g->has_model, dset, gset, n, mixed,
+                       tiled_plan_side(g, flags, n, &side));
   if (!pl.ok) return Status::ok();
   *used = true;
   StreamPrep prep;
@@ -263,7 +275,7 @@ Status linear_op_stream(hpgb_gridder* g, const void* d_vis, size_t n, int op,
   CFShape cf;
   cf.add(g);
   const StreamPlan pl =
-      make_stream_plan(g, cf, gather, !gather, gather, set, set, n, false);
+      make_stream_plan(g, cf, gather, !gather, gather, set, set, n, false, true);
   if (!pl.ok) return Status::ok();
   *used = true;
   StreamPrep prep;

@@ -28,13 +28,14 @@ struct CFShape {
 
 // The plan of a launch over nvis visibilities with g's polarizations and
 // Mueller tables.  dset, gset: the degridding and gridding index tables for
-// w <= 0 and w > 0.  tiles_fp32: the tiled kernel would take FP32 tiles.  Not
-// ok where another kernel is the faster one, or the only one.
+// w <= 0 and w > 0.  tiles_fp32: the tiled kernel would take FP32 tiles;
+// tiled_takes: it (or the tiled operators) can take the batch.  Not ok where
+// another kernel is the faster one, or the only one.
 StreamPlan make_stream_plan(const hpgb_gridder* g, const CFShape& cf,
                             bool degrid, bool grid, bool has_model,
                             const int (*const dset[2])[4],
                             const int (*const gset[2])[4], size_t nvis,
-                            bool tiles_fp32);
+                            bool tiles_fp32, bool tiled_takes);
 
 // whether a batch's visibilities are put into tile order
 bool stream_sorted(const hpgb_gridder* g, size_t n, bool has_model);

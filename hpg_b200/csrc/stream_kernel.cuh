@@ -48,9 +48,11 @@ namespace stream {
 constexpr int kWarps = 16;      // ring
 constexpr int kFreeWarps = 8;   // no ring
 constexpr int kProducers = 2;
-constexpr int warps_of(bool ring) { return ring ? kWarps : kFreeWarps; }
-constexpr int ctas_per_sm(bool ring, int npol) {
-  return ring ? 1 : npol == 1 ? 3 : 2;
+constexpr int warps_of(bool ring, int W) {
+  return ring || W > kFreeWarps ? kWarps : kFreeWarps;
+}
+constexpr int ctas_per_sm(bool ring, int npol, int W) {
+  return ring || W > kFreeWarps ? 1 : npol == 1 ? 3 : 2;
 }
 constexpr int kSlots = 32;      // visibilities in flight (ring)
 constexpr int kMaxRuns = 8;
@@ -139,6 +141,17 @@ struct CFRef {
       return __ldg(at + off);
   }
 };
+
+// a row's CF values at one cell; o: the row's plane offsets (-1: inactive)
+template <int N, bool RING>
+__device__ __forceinline__ void row_planes(const CFRef<RING>& cf, const int* o,
+                                           bool dense, float2 (&v)[N]) {
+  const int4 o4 = *reinterpret_cast<const int4*>(o);
+  const int off[4] = {o4.x, o4.y, o4.z, o4.w};
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    if (dense || off[k] >= 0) v[k] = cf.plus(off[k]).get(0);
+}
 
 // exp(i (phi_x(X) + phi_y(Y))) from the group's table of the two axes'
 // phasors: taps_x + taps_y sine-cosine pairs per visibility instead of two
@@ -277,11 +290,12 @@ struct Products {
 // last job's ended.
 
 template <int N, bool DIAG, int FORM, int W, bool RING>
-__global__ void __launch_bounds__(32 * warps_of(RING), ctas_per_sm(RING, N))
+__global__ void __launch_bounds__(32 * warps_of(RING, W),
+                                  ctas_per_sm(RING, N, W))
 stream_kernel(const __grid_constant__ StreamParams p) {
   using V = typename Sums<N, FORM>::V;  // model element
   using G = typename std::conditional<FORM == kLinear, double2, float2>::type;
-  constexpr int kCompute = RING ? kWarps - kProducers : kFreeWarps;
+  constexpr int kCompute = RING ? kWarps - kProducers : warps_of(false, W);
   constexpr int kG = kCompute / W;  // groups
   constexpr int kT = 32 * W;        // threads of a group
   constexpr int NV = 2 * N;
@@ -566,7 +580,8 @@ stream_kernel(const __grid_constant__ StreamParams p) {
             Sums<N, FORM> sum;
             sum.zero();
             // kU cells at a time, their model values asked for together
-            constexpr int kU = DIAG ? 4 : 2;
+            constexpr bool kAll = !DIAG && !RING;
+            constexpr int kU = DIAG ? 4 : kAll ? 1 : 2;
             constexpr int kRows = DIAG ? N : 4;
             int chain = 0;
             for (int c0 = gt; c0 < ncell; c0 += kU * kT) {
@@ -609,6 +624,23 @@ stream_kernel(const __grid_constant__ StreamParams p) {
                 }
               }
               const CFRef<RING> cfc = cfb.plus(c0);
+              if constexpr (kAll) {
+                // a row's CF values ahead of its products
+                float2 cf[2][N];
+                row_planes<N, RING>(cfc, offs, p.dense, cf[0]);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                  if (r >= p.nrow) break;
+                  if (r + 1 < 4 && r + 1 < p.nrow)
+                    row_planes<N, RING>(cfc, offs + 4 * (r + 1), p.dense,
+                                        cf[(r + 1) & 1]);
+#pragma unroll
+                  for (int v = 0; v < N; ++v)
+                    if (p.dense || offs[4 * r + v] >= 0)
+                      sum.add(v, cf[r & 1][v], m[0][r], pos_w);
+                }
+                continue;
+              }
 #pragma unroll
               for (int r = 0; r < kRows; ++r) {
                 if (!DIAG && r >= p.nrow) break;
@@ -758,6 +790,7 @@ stream_kernel(const __grid_constant__ StreamParams p) {
             for (int w0 = wig * 32; w0 < ncell; w0 += kU * kT) {
               uint32_t at_a[kU], at_b[kU];
               float2 cfd[kU][DIAG ? N : 1];
+              constexpr bool kAll = !DIAG && !RING;
 #pragma unroll
               for (int u = 0; u < kU; ++u) {
                 const int ca = w0 + u * kT + (lane >> 1), c = ca + 16 * h;
@@ -787,6 +820,9 @@ stream_kernel(const __grid_constant__ StreamParams p) {
                                     pos_w ? -__double2float_rn(sc.y)
                                           : __double2float_rn(sc.y));
                 }
+                float2 cfr[2][N];  // a row's CF values ahead of its products
+                if constexpr (kAll)
+                  if (on) row_planes<N, RING>(cfb.plus(c), offs + 16, p.dense, cfr[0]);
                 double* dst_a = gbase + 2 * size_t(at_a[u]);
                 double* dst_b = gbase + 2 * size_t(at_b[u]);
 #pragma unroll
@@ -796,6 +832,16 @@ stream_kernel(const __grid_constant__ StreamParams p) {
                   pr.zero();
                   if constexpr (DIAG) {
                     pr.add(cfd[u][r], gv[r], screen, scf);
+                  } else if constexpr (kAll) {
+                    if (on) {
+                      if (r + 1 < 4 && r + 1 < p.nrow)
+                        row_planes<N, RING>(cfb.plus(c), offs + 20 + 4 * r,
+                                            p.dense, cfr[(r + 1) & 1]);
+#pragma unroll
+                      for (int v = 0; v < N; ++v)
+                        if (p.dense || offs[16 + 4 * r + v] >= 0)
+                          pr.add(cfr[r & 1][v], gv[v], screen, scf);
+                    }
                   } else {
                     const int4 o4 =
                         *reinterpret_cast<const int4*>(offs + 16 + 4 * r);

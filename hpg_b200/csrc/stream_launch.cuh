@@ -20,7 +20,8 @@ Status launch_variant(hpgb_gridder* g, const StreamPlan& pl,
     HPGB_CUDA_TRY(cudaEventCreate(&ev[1]));
     HPGB_CUDA_TRY(cudaEventRecord(ev[0], g->stream));
   }
-  kern<<<unsigned(pl.ctas), 32 * warps_of(RING), size_t(pl.smem), g->stream>>>(p);
+  kern<<<unsigned(pl.ctas), 32 * warps_of(RING, W), size_t(pl.smem),
+         g->stream>>>(p);
   HPGB_CUDA_TRY(cudaGetLastError());
   ++g->launches;
   if (g->profile) {
@@ -43,8 +44,9 @@ Status launch_variants(hpgb_gridder* g, const StreamPlan& pl,
   } else if (pl.ring) {
     if (pl.warps == 7) return launch_variant<N, false, FORM, 7, true>(g, pl, p);
     if (pl.warps == 2) return launch_variant<N, false, FORM, 2, true>(g, pl, p);
-  } else if (pl.warps == 1) {
-    return launch_variant<N, false, FORM, 1, false>(g, pl, p);
+  } else {
+    if (pl.warps == 16) return launch_variant<N, false, FORM, 16, false>(g, pl, p);
+    if (pl.warps == 1) return launch_variant<N, false, FORM, 1, false>(g, pl, p);
   }
   return Status::err(HPGB_ERROR_OTHER, "stream kernel variant missing");
 }

@@ -1,6 +1,6 @@
 """The automatic choice's one-visibility-per-group kernel (stream_kernel.cuh)
 against the per-visibility kernels (HPGB_KERNEL_DIRECT), which the parity
-tests pin to the oracle, at the edges of its variants: one, two and four warps
+tests pin to the oracle, at the edges of its variants: one to sixteen warps
 per visibility, CF slices from global memory and through the ring (which wraps
 and holds a single part), partial Mueller rows, several cubes, footprints off
 the grid, batches that end inside a CTA's block.
@@ -44,6 +44,7 @@ CASES = {
                     [-1, -1, -1, -1]], False, (4, 8), 1203, 0.2),
     "ring-two-warps": (4, dense(4), False, (8, 12, 16), 1999, 0.2),
     "ring-seven-warps": (4, dense(4), False, (8, 24, 36), 1013, None),
+    "sixteen-warps": (4, dense(4), False, (9, 52), 207, 0.2),
 }
 
 
