@@ -579,13 +579,16 @@ stream_kernel(const __grid_constant__ StreamParams p) {
             const V* model = static_cast<const V*>(job.model) + org;
             Sums<N, FORM> sum;
             sum.zero();
-            // kU cells at a time, their model values asked for together
+            // kU cells at a time, their model values asked for together (two
+            // polarizations, supports 8 to 64, 500k visibilities, mixed: 2.8
+            // ms with four, 2.4 with six; asking for the next step's CF values
+            // too: 3.4, two steps' registers leave too few)
             constexpr bool kAll = !DIAG && !RING;
-            constexpr int kU = DIAG ? 4 : kAll ? 1 : 2;
+            constexpr int kU = DIAG ? (FORM == kMixed && N == 2 ? 6 : 4) : kAll ? 1 : 2;
             constexpr int kRows = DIAG ? N : 4;
             int chain = 0;
             for (int c0 = gt; c0 < ncell; c0 += kU * kT) {
-              if (chain == 16 / kU) {
+              if (chain == (16 + kU - 1) / kU) {
                 sum.settle();
                 chain = 0;
               }
@@ -785,7 +788,7 @@ stream_kernel(const __grid_constant__ StreamParams p) {
             double* const gbase = reinterpret_cast<double*>(job.grid + org) + h;
             // kU steps of 32 cells at a time, their CF values asked for
             // together
-            constexpr int kU = DIAG ? (N <= 2 ? 4 : 2) : (N <= 2 ? 2 : 1);
+            constexpr int kU = DIAG ? (N == 1 ? 4 : N == 2 ? 6 : 2) : (N <= 2 ? 2 : 1);
             constexpr int kRows = DIAG ? N : 4;
             for (int w0 = wig * 32; w0 < ncell; w0 += kU * kT) {
               uint32_t at_a[kU], at_b[kU];
