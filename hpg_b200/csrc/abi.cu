@@ -473,6 +473,20 @@ int hpgb_grid_visibilities(hpgb_gridder* g, const void* vis, size_t n,
     HPGB_CUDA_TRY(cudaSetDevice(g->device));
     const size_t rec = visdata_size(npol);
     const size_t bytes = n * rec;
+    if (vis_on_device) {
+      bool used = false;
+      HPGB_TRY(grid_stream_device(
+          g, vis, n, flags,
+          (flags & HPGB_RETURN_VISIBILITIES) ? returned : nullptr, &used));
+      if (used) {
+        if (flags & HPGB_RETURN_VISIBILITIES) {
+          g->pending_dst = returned;
+          g->pending_bytes = bytes;
+          g->pending_on_device = true;
+        }
+        return Status::ok();
+      }
+    }
     // A host batch outside a stream capture is copied on the copy stream
     // into the staging buffer not used by the previous call, so that the
     // copy overlaps the previous call's work (the work on the gridder's

@@ -13,18 +13,9 @@ namespace hpgb {
 
 Status grid_batch(hpgb_gridder* g, const void* d_vis, size_t n,
                   unsigned flags) {
-  // the automatic choice, unless the tiled kernel's plan was set by hand
-  if (g->kernel_kind == HPGB_KERNEL_AUTO && g->tplan.ring_parts == 0 &&
-      g->tplan.chunk_vis == 0 && g->tplan.tile_side == 0) {
-    bool used = false;
-    HPGB_TRY(grid_stream(g, const_cast<void*>(d_vis), n, flags, &used));
-    if (used) {
-      int side = 0;
-      g->last_kernel = tiled_plan_side(g, flags, n, &side) ? HPGB_KERNEL_TILED
-                                                           : HPGB_KERNEL_DIRECT;
-      return Status::ok();
-    }
-  }
+  bool streamed = false;
+  HPGB_TRY(grid_stream(g, const_cast<void*>(d_vis), n, flags, &streamed));
+  if (streamed) return Status::ok();
   if (g->kernel_kind != HPGB_KERNEL_DIRECT) {
     bool used = false;
     HPGB_TRY(grid_tiled(g, const_cast<void*>(d_vis), n, flags, &used));

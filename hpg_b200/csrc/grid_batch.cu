@@ -274,7 +274,8 @@ Status grid_batch_stream(hpgb_gridder* const* gs, size_t njobs,
     if (js != st) HPGB_CUDA_TRY(cudaStreamWaitEvent(js, fork, 0));
     StreamPrep prep;
     HPGB_TRY(prepare_stream(g, d_vis[j], nvis[j],
-                            stream_sorted(g, nvis[j], model), &prep, js));
+                            stream_sorted(g, nvis[j], model), degrid, grid, false,
+                            &prep, js));
     if (model && mixed) HPGB_TRY(tiled::ensure_model32(g, js));
     StreamJob& b = table->jobs[table->njobs++];
     b.descs = prep.descs;
@@ -306,6 +307,7 @@ Status grid_batch_stream(hpgb_gridder* const* gs, size_t njobs,
   p.njobs = table->njobs;
   p.update_weights = (flags & HPGB_UPDATE_GRID_WEIGHTS) != 0;
   p.rec_stride = int(visdata_size(g0->npol));
+  p.write_back = 1;
   p.status = vb.counters.as<unsigned>();
   p.wait_limit_ns = g0->wait_limit_ns;
   return launch_stream(g0, mixed ? stream::kMixed : stream::kFP64, pl, p);

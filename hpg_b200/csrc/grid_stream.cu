@@ -159,7 +159,8 @@ StreamPlan make_stream_plan(const hpgb_gridder* g, const CFShape& cf,
       if (tiled_takes) return pl;
       pl.ring = false;
       pl.warps = 16;
-    } else if (pl.ring && part > 48 * 1024 && nvis > 4000) {
+    } else if (pl.ring && part > 48 * 1024 &&
+               nvis > size_t(tiles_fp32 || use_g ? 6000 : 3000)) {
       return pl;
     }
   }
@@ -191,8 +192,14 @@ StreamPlan make_stream_plan(const hpgb_gridder* g, const CFShape& cf,
       }
   p.evict_first = cf.table_bytes > size_t(96) << 20;
   pl.ctas = sms * ctas_per_sm(pl.ring, n, pl.warps);
-  p.block_vis = int(std::min<size_t>(
-      kBlockVis, std::max<size_t>(1, (nvis + pl.ctas - 1) / size_t(pl.ctas))));
+  // whole rounds of blocks over the CTAs, several where there are
+  // visibilities for it, so that the CTAs end level
+  const size_t per_cta = (nvis + pl.ctas - 1) / size_t(pl.ctas);
+  const size_t most = pl.ring ? kBlockVis : kFreeBlockVis;
+  const size_t rounds = std::max<size_t>(per_cta >= 64 ? 4 : 1,
+                                         (per_cta + most - 1) / most);
+  p.block_vis = int(std::max<size_t>(
+      1, (nvis + pl.ctas * rounds - 1) / (pl.ctas * rounds)));
   pl.ok = true;
   return pl;
 }
@@ -218,8 +225,12 @@ Status launch_stream(hpgb_gridder* g, int form, const StreamPlan& pl,
 
 using namespace stream;
 
-Status grid_stream(hpgb_gridder* g, void* d_vis, size_t n, unsigned flags,
-                   bool* used) {
+// in_place: the records are the caller's, read where they lie; with `returned`
+// they are copied there first and their values written there, without nothing
+// is written back.
+static Status grid_stream_run(hpgb_gridder* g, void* d_vis, size_t n,
+                              unsigned flags, bool in_place, void* returned,
+                              bool* used) {
   *used = false;
   const bool degrid = flags & HPGB_DO_DEGRID, grid = flags & HPGB_DO_GRID;
   if (n == 0 || n > size_t(0x7fffffff) || !(degrid || grid))
@@ -235,15 +246,22 @@ Status grid_stream(hpgb_gridder* g, void* d_vis, size_t n, unsigned flags,
   CFShape cf;
   cf.add(g);
   int side = 0;
+  const bool tiled = tiled_plan_side(g, flags, n, &side);
   const StreamPlan pl =
       make_stream_plan(g, cf, degrid, grid, g->has_model, dset, gset, n, mixed,
-                       tiled_plan_side(g, flags, n, &side));
+                       tiled);
   if (!pl.ok) return Status::ok();
   *used = true;
+  g->last_kernel = tiled ? HPGB_KERNEL_TILED : HPGB_KERNEL_DIRECT;
+  if (in_place && returned && returned != d_vis) {
+    HPGB_CUDA_TRY(cudaMemcpyAsync(returned, d_vis, n * visdata_size(g->npol),
+                                  cudaMemcpyDeviceToDevice, g->stream));
+    d_vis = returned;
+  }
   StreamPrep prep;
   HPGB_TRY(prepare_stream(g, d_vis, n,
-                          stream_sorted(g, n, degrid && g->has_model), &prep,
-                          g->stream));
+                          stream_sorted(g, n, degrid && g->has_model), degrid,
+                          grid, false, &prep, g->stream));
   if (mixed && degrid && g->has_model)
     HPGB_TRY(tiled::ensure_model32(g, g->stream));
   StreamParams p = pl.p;
@@ -259,9 +277,34 @@ Status grid_stream(hpgb_gridder* g, void* d_vis, size_t n, unsigned flags,
   p.job.ny = int(g->grid_size[1]);
   p.update_weights = (flags & HPGB_UPDATE_GRID_WEIGHTS) != 0;
   p.rec_stride = int(visdata_size(g->npol));
+  p.write_back = !in_place || returned;
   p.status = g->vb.counters.as<unsigned>();
   p.wait_limit_ns = g->wait_limit_ns;
   return launch_stream(g, mixed ? kMixed : kFP64, pl, p);
+}
+
+// the automatic choice, unless the tiled kernel's plan was set by hand
+static bool automatic(const hpgb_gridder* g) {
+  return g->kernel_kind == HPGB_KERNEL_AUTO && g->tplan.ring_parts == 0 &&
+         g->tplan.chunk_vis == 0 && g->tplan.tile_side == 0;
+}
+
+Status grid_stream(hpgb_gridder* g, void* d_vis, size_t n, unsigned flags,
+                   bool* used) {
+  *used = false;
+  if (!automatic(g)) return Status::ok();
+  return grid_stream_run(g, d_vis, n, flags, false, nullptr, used);
+}
+
+Status grid_stream_device(hpgb_gridder* g, const void* vis, size_t n,
+                          unsigned flags, void* returned, bool* used) {
+  *used = false;
+  // (a copy takes records at any address, the kernels want them aligned)
+  if (!automatic(g) || reinterpret_cast<uintptr_t>(vis) % 8 != 0 ||
+      (returned && reinterpret_cast<uintptr_t>(returned) % 8 != 0))
+    return Status::ok();
+  return grid_stream_run(g, const_cast<void*>(vis), n, flags, true, returned,
+                         used);
 }
 
 Status linear_op_stream(hpgb_gridder* g, const void* d_vis, size_t n, int op,
@@ -279,8 +322,9 @@ Status linear_op_stream(hpgb_gridder* g, const void* d_vis, size_t n, int op,
   if (!pl.ok) return Status::ok();
   *used = true;
   StreamPrep prep;
-  HPGB_TRY(prepare_stream(g, const_cast<void*>(d_vis), n,
-                          stream_sorted(g, n, false), &prep, g->stream));
+  HPGB_TRY(prepare_stream(g, d_vis, n,
+                          stream_sorted(g, n, false), gather, !gather, true,
+                          &prep, g->stream));
   StreamParams p = pl.p;
   p.op = op;
   p.job.descs = prep.descs;

@@ -146,15 +146,18 @@ __global__ void chunk_write_kernel(const unsigned* counts,
   if (t == ntiles - 1) *num_chunks = cstart[t] + nch[t];
 }
 
-// the descriptor and slice reference of visibility i (on the grid at vc), its
-// footprint origin relative to (x0, y0)
+// The descriptor and slice reference of visibility i (on the grid at vc), its
+// footprint origin relative to (x0, y0).  what: the fields the launch reads
+// beside the geometry (FP64 divisions and magnitudes are what this costs: an
+// 11 us chain for a small batch); the others stay zero.
+enum : int { kWantFactor = 1, kWantWeights = 2, kWantScaled = 4, kWantAll = 7 };
 template <int N>
 __device__ __forceinline__ void make_desc(const VisData<N>& vd, unsigned i,
                                           const VisCoord& vc, int x0, int y0,
                                           const GridGeom& g,
                                           const CFGroup* groups,
-                                          const float2* cf_base, TileDesc& d,
-                                          SliceRef& s) {
+                                          const float2* cf_base, int what,
+                                          TileDesc& d, SliceRef& s) {
   const CFGroup& G = groups[vc.grp];
   d.index = int(i);
   d.cx = int16_t(vc.grid_coord[0] - x0);
@@ -179,19 +182,21 @@ __device__ __forceinline__ void make_desc(const VisData<N>& vd, unsigned i,
   for (int v = 0; v < 4; ++v) {
     d.vals[v] = v < N ? vd.vis[v] : make_float2(0.f, 0.f);
     d.weights[v] = v < N ? vd.weights[v] : 0.f;
-    d.gvis[v] = v < N ? scale_for_gridding(vd.vis[v], d.phasor, vd.weights[v])
-                      : make_float2(0.f, 0.f);
+    d.gvis[v] = v < N && (what & kWantScaled)
+                    ? scale_for_gridding(vd.vis[v], d.phasor, vd.weights[v])
+                    : make_float2(0.f, 0.f);
+    d.wfac[v] = make_double2(0.0, 0.0);
+    if (v >= N || !(what & kWantFactor)) continue;
     // normaliser: sum over grid rows of the slice sums, conjugated for
     // non-positive w (src/hpg_core.hpp:598-600, :659-661)
     double2 den = make_double2(0.0, 0.0);
-    if (v < N)
-      for (int r = 0; r < g.nrow; ++r) {
-        const int m = dmi[r][v];
-        if (m >= 0) {
-          const double2 w = ws[m];
-          den = cadd_d(den, make_double2(w.x, vc.pos_w ? w.y : -w.y));
-        }
+    for (int r = 0; r < g.nrow; ++r) {
+      const int m = dmi[r][v];
+      if (m >= 0) {
+        const double2 w = ws[m];
+        den = cadd_d(den, make_double2(w.x, vc.pos_w ? w.y : -w.y));
       }
+    }
     // prediction = sum * conj(phasor) / normaliser (src/hpg_core.hpp:670-679),
     // with the factor formed here once per visibility
     if (den.x == 0.0 && den.y == 0.0) den = make_double2(1.0, 0.0);
@@ -200,7 +205,7 @@ __device__ __forceinline__ void make_desc(const VisData<N>& vd, unsigned i,
   // grid weight per row: sum_vpol |sum_XY cf| * w (src/hpg_core.hpp:877-885)
   for (int r = 0; r < 4; ++r) {
     double tw = 0.0;
-    if (r < g.nrow)
+    if (r < g.nrow && (what & kWantWeights))
       for (int v = 0; v < N; ++v) {
         const int m = gmi[r][v];
         if (m >= 0) {
@@ -243,7 +248,8 @@ __global__ void tile_desc_kernel(const VisData<N>* vis, const unsigned* order,
   const int ty = int((key / unsigned(tg.ntx)) % unsigned(tg.nty));
   TileDesc d;
   SliceRef s;
-  make_desc<N>(vd, i, vc, tx * tg.T, ty * tg.T, g, groups, cf_base, d, s);
+  make_desc<N>(vd, i, vc, tx * tg.T, ty * tg.T, g, groups, cf_base, kWantAll, d,
+               s);
   descs[pidx] = d;
   srefs[pidx] = s;
 }
@@ -279,7 +285,8 @@ template <int N>
 __global__ void stream_desc_kernel(const VisData<N>* vis, const unsigned* order,
                                    size_t n, GridGeom g, const CFGroup* groups,
                                    const float2* cf_base, TileDesc* descs,
-                                   SliceRef* srefs, unsigned* num_vis) {
+                                   SliceRef* srefs, unsigned* num_vis,
+                                   int what) {
   const size_t pidx = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
   if (!order && pidx == 0) *num_vis = unsigned(n);
   if (pidx >= (order ? size_t(*num_vis) : n)) return;
@@ -292,7 +299,7 @@ __global__ void stream_desc_kernel(const VisData<N>* vis, const unsigned* order,
   SliceRef s;
   if (vc.in_grid) {
     make_desc<N>(vd, i, vc, vc.grid_coord[0], vc.grid_coord[1], g, groups,
-                 cf_base, d, s);
+                 cf_base, what, d, s);
     descs[pidx] = d;
   } else {
     // (a slice of one 16-byte unit per plane, never used)
@@ -701,8 +708,9 @@ Status grid_tiled_n(hpgb_gridder* g, void* d_vis, size_t n, unsigned flags,
 namespace {
 
 template <int N>
-Status prepare_stream_n(hpgb_gridder* g, void* d_vis, size_t n, bool sorted,
-                        StreamPrep* out, cudaStream_t st) {
+Status prepare_stream_n(hpgb_gridder* g, const void* d_vis, size_t n,
+                        bool sorted, int what, StreamPrep* out,
+                        cudaStream_t st) {
   VisBuffers& vb = g->vb;
   const GridGeom geom = g->geom();
   const CFGroup* groups = g->cf.desc.as<const CFGroup>();
@@ -742,7 +750,7 @@ Status prepare_stream_n(hpgb_gridder* g, void* d_vis, size_t n, bool sorted,
   }
   stream_desc_kernel<N><<<blocks, 256, 0, st>>>(
       vis, order, n, geom, groups, g->cf.data.as<const float2>(), descs, srefs,
-      num_vis);
+      num_vis, what);
   HPGB_CUDA_TRY(cudaGetLastError());
   ++g->launches;
   *out = StreamPrep{descs, srefs, num_vis};
@@ -751,13 +759,17 @@ Status prepare_stream_n(hpgb_gridder* g, void* d_vis, size_t n, bool sorted,
 
 }  // namespace
 
-Status prepare_stream(hpgb_gridder* g, void* d_vis, size_t n, bool sorted,
+Status prepare_stream(hpgb_gridder* g, const void* d_vis, size_t n,
+                      bool sorted, bool degrid, bool grid, bool linear,
                       StreamPrep* out, cudaStream_t st) {
+  const int what =
+      linear ? kWantFactor
+             : (degrid ? kWantFactor : kWantScaled) | (grid ? kWantWeights : 0);
   switch (g->npol) {
-    case 1: return prepare_stream_n<1>(g, d_vis, n, sorted, out, st);
-    case 2: return prepare_stream_n<2>(g, d_vis, n, sorted, out, st);
-    case 3: return prepare_stream_n<3>(g, d_vis, n, sorted, out, st);
-    case 4: return prepare_stream_n<4>(g, d_vis, n, sorted, out, st);
+    case 1: return prepare_stream_n<1>(g, d_vis, n, sorted, what, out, st);
+    case 2: return prepare_stream_n<2>(g, d_vis, n, sorted, what, out, st);
+    case 3: return prepare_stream_n<3>(g, d_vis, n, sorted, what, out, st);
+    case 4: return prepare_stream_n<4>(g, d_vis, n, sorted, what, out, st);
     default: return Status::err(HPGB_ERROR_OTHER, "bad polarization count");
   }
 }

@@ -140,10 +140,14 @@ Status copy_cf(hpgb_gridder* dst, const hpgb_gridder* src);
 Status grid_tiled(hpgb_gridder* g, void* d_vis, size_t n, unsigned flags,
                   bool* used);
 
-// grid_stream.cu: one visibility per group of warps, straight into the grid;
-// *used is false when it cannot take the batch
+// grid_stream.cu: one visibility per group of warps, straight into the grid,
+// where that is the automatic choice; *used is false when it is not
 Status grid_stream(hpgb_gridder* g, void* d_vis, size_t n, unsigned flags,
                    bool* used);
+// the same on the caller's device records, without the gridder's copy of
+// them; values are written to `returned` (which may be vis), or nowhere
+Status grid_stream_device(hpgb_gridder* g, const void* vis, size_t n,
+                          unsigned flags, void* returned, bool* used);
 
 // grid_tiled.cu: the uv tile side of the plan the tiled kernel would take
 // for the batch (false when no plan fits)

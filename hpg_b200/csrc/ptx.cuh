@@ -211,6 +211,11 @@ __device__ __forceinline__ void sts_d2(uint32_t a, double2 v) {
 }
 
 
+// a line of global memory into L1 (no effect on what is read)
+__device__ __forceinline__ void prefetch_l1(const void* p) {
+  asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
+}
+
 // bulk copy global -> this CTA's shared memory, completion counted in bytes
 // on bar; dst, src and bytes are 16-byte multiples
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src,

@@ -57,6 +57,7 @@ constexpr int ctas_per_sm(bool ring, int npol, int W) {
 constexpr int kSlots = 32;      // visibilities in flight (ring)
 constexpr int kMaxRuns = 8;
 constexpr int kBlockVis = 16;   // consecutive visibilities a CTA takes, at most
+constexpr int kFreeBlockVis = 64;  // without the ring
 
 enum Form : int { kFP64 = 0, kMixed = 1, kLinear = 2 };
 
@@ -79,6 +80,7 @@ struct StreamParams {
   int njobs;
   int nrow, ncube;
   int do_degrid, do_grid, update_weights, has_model;
+  int write_back;   // predictions or residuals go into the records
   int rec_stride;
   // slot planes (ring) or Mueller planes (no ring) of each row's elements
   // for w <= 0 and w > 0, a signed byte per element (-1: inactive); with one
@@ -509,8 +511,9 @@ stream_kernel(const __grid_constant__ StreamParams p) {
         const unsigned i0 = b * bv;
         const int count = int(min(bv, n - i0));
         // (groups take visibilities in turn by q, so that they stay level)
-        for (int k = int((uint32_t(grp) + kG - q % kG) % kG); k < count;
-             k += kG) {
+        const int k0 = int((uint32_t(grp) + kG - q % kG) % kG);
+        long long next_off = 0;
+        for (int k = k0; k < count; k += kG) {
           const uint32_t qq = q + uint32_t(k);
           const int s = int(qq % uint32_t(kSlots));
           const TileDesc* d;
@@ -535,7 +538,18 @@ stream_kernel(const __grid_constant__ StreamParams p) {
           } else {
             group_sync();  // the last visibility's readers of part and tab
             d = job.descs + i0 + k;
-            cfb.at = job.cf + job.srefs[i0 + k].off;
+            cfb.at = job.cf + (k == k0 ? job.srefs[i0 + k].off : next_off);
+            // the group's next visibility of the block: its descriptor, and
+            // the start of its CF slice, into L1 meanwhile
+            if (k + kG < count) {
+              const SliceRef sr = job.srefs[i0 + k + kG];
+              next_off = sr.off;
+              if (gt < 8)
+                ptx::prefetch_l1(reinterpret_cast<const char*>(d + kG) + 32 * gt);
+              else if (gt < 32 && 128 * (gt - 8) < p.nplanes * sr.pstride * 8)
+                ptx::prefetch_l1(reinterpret_cast<const char*>(job.cf + next_off) +
+                                 128 * (gt - 8));
+            }
           }
           const int4 head4 = *reinterpret_cast<const int4*>(d);
           const int tx = head4.z & 0xff, ty = (head4.z >> 8) & 0xff;
@@ -751,9 +765,9 @@ stream_kernel(const __grid_constant__ StreamParams p) {
                 const float2 val = d->vals[lane];
                 const float2 rr = make_float2(__fsub_rn(val.x, pred.x),
                                               __fsub_rn(val.y, pred.y));
-                if (wig == 0) out[lane] = rr;
+                if (wig == 0 && p.write_back) out[lane] = rr;
                 gout = scale_for_gridding(rr, phasor, d->weights[lane]);
-              } else if (wig == 0) {
+              } else if (wig == 0 && p.write_back) {
                 out[lane] = pred;
               }
             } else {

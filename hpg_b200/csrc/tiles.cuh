@@ -105,14 +105,16 @@ Status prepare_tiles(hpgb_gridder* g, void* d_vis, size_t n, int T, int ntx,
 // (stream_kernel.cuh): descriptors and slice references in the order of uv
 // tiles of kStreamTile cells, or as in the batch (visibilities off the grid
 // flagged kSkip) when sorted is false.  num_vis: device word, the descriptors
-// to take.
+// to take.  degrid, grid, linear: the passes (or linear operator) whose
+// fields the descriptors need.
 constexpr int kStreamTile = 64;
 struct StreamPrep {
   const TileDesc* descs;
   const SliceRef* srefs;
   const unsigned* num_vis;
 };
-Status prepare_stream(hpgb_gridder* g, void* d_vis, size_t n, bool sorted,
+Status prepare_stream(hpgb_gridder* g, const void* d_vis, size_t n,
+                      bool sorted, bool degrid, bool grid, bool linear,
                       StreamPrep* out, cudaStream_t st);
 
 }  // namespace hpgb
