@@ -291,7 +291,9 @@ struct Products {
 // them uneven: measured up to 1.4x slower), each job's first one where the
 // last job's ended.
 
-template <int N, bool DIAG, int FORM, int W, bool RING>
+// PASS: 1 degrids, 2 grids, 3 does both (kernels of their own: one with the
+// passes as flags keeps the registers of both), 0: as p says.
+template <int N, bool DIAG, int FORM, int W, bool RING, int PASS>
 __global__ void __launch_bounds__(32 * warps_of(RING, W),
                                   ctas_per_sm(RING, N, W))
 stream_kernel(const __grid_constant__ StreamParams p) {
@@ -341,9 +343,12 @@ stream_kernel(const __grid_constant__ StreamParams p) {
     }
     __syncthreads();
   }
-  const bool degrid = p.do_degrid && p.has_model;
+  const bool degrid = PASS == 2 ? false
+                      : PASS == 3 ? true
+                                  : p.do_degrid && p.has_model;
+  const bool do_grid = PASS ? PASS >= 2 : bool(p.do_grid);
   const int njobs = p.jobs ? p.njobs : 1;
-  const bool cf_needed = degrid || p.do_grid;
+  const bool cf_needed = degrid || do_grid;
 
   if (RING && warp >= kCompute) {
     // ---------------- producer warps ----------------
@@ -577,7 +582,7 @@ stream_kernel(const __grid_constant__ StreamParams p) {
           }
           double2 lin_in = make_double2(0.0, 0.0);
           if constexpr (FORM == kLinear)
-            if (p.do_grid)
+            if (do_grid)
               lin_in = __ldg(p.vals_in + size_t(head4.x) * N + vl);
           if (screen && cf_needed) {
             for (int i = gt; i < tx + ty; i += kT) {
@@ -601,6 +606,7 @@ stream_kernel(const __grid_constant__ StreamParams p) {
             constexpr int kU = DIAG ? (FORM == kMixed && N == 2 ? 6 : 4) : kAll ? 1 : 2;
             constexpr int kRows = DIAG ? N : 4;
             int chain = 0;
+#pragma unroll 1
             for (int c0 = gt; c0 < ncell; c0 += kU * kT) {
               if (chain == (16 + kU - 1) / kU) {
                 sum.settle();
@@ -737,7 +743,7 @@ stream_kernel(const __grid_constant__ StreamParams p) {
           if constexpr (FORM == kLinear) {
             const double wgt = double(d->weights[vl]);
             const double2 wfac = d->wfac[vl];
-            if (p.do_grid) {
+            if (do_grid) {
               // D^H: phasor / conj(den) = conj(conj(phasor) / den);
               // G: phasor * w
               gout = cmul_d(p.op == 1 ? make_double2(wfac.x, -wfac.y)
@@ -761,7 +767,7 @@ stream_kernel(const __grid_constant__ StreamParams p) {
               }
               float2* out = reinterpret_cast<float2*>(
                   job.records + size_t(head4.x) * p.rec_stride);
-              if (p.do_grid) {
+              if (do_grid) {
                 const float2 val = d->vals[lane];
                 const float2 rr = make_float2(__fsub_rn(val.x, pred.x),
                                               __fsub_rn(val.y, pred.y));
@@ -774,7 +780,7 @@ stream_kernel(const __grid_constant__ StreamParams p) {
               gout = d->gvis[lane];
             }
           }
-          if (p.do_grid) {
+          if (do_grid) {
             if (wig == 0) {
               if (cube != wcube) {
                 flush_weights();
@@ -804,6 +810,7 @@ stream_kernel(const __grid_constant__ StreamParams p) {
             // together
             constexpr int kU = DIAG ? (N == 1 ? 4 : N == 2 ? 6 : 2) : (N <= 2 ? 2 : 1);
             constexpr int kRows = DIAG ? N : 4;
+#pragma unroll 1
             for (int w0 = wig * 32; w0 < ncell; w0 += kU * kT) {
               uint32_t at_a[kU], at_b[kU];
               float2 cfd[kU][DIAG ? N : 1];

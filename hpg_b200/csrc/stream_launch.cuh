@@ -8,10 +8,10 @@
 namespace hpgb {
 namespace stream {
 
-template <int N, bool DIAG, int FORM, int W, bool RING>
-Status launch_variant(hpgb_gridder* g, const StreamPlan& pl,
+template <int N, bool DIAG, int FORM, int W, bool RING, int PASS>
+Status launch_pass(hpgb_gridder* g, const StreamPlan& pl,
                       const StreamParams& p) {
-  auto kern = stream_kernel<N, DIAG, FORM, W, RING>;
+  auto kern = stream_kernel<N, DIAG, FORM, W, RING, PASS>;
   HPGB_CUDA_TRY(cudaFuncSetAttribute(
       kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem));
   cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -29,6 +29,24 @@ Status launch_variant(hpgb_gridder* g, const StreamPlan& pl,
     g->prof_events.emplace_back(ev[0], ev[1]);
   }
   return Status::ok();
+}
+
+template <int N, bool DIAG, int FORM, int W, bool RING>
+Status launch_variant(hpgb_gridder* g, const StreamPlan& pl,
+                      const StreamParams& p) {
+  if constexpr (DIAG) {
+    // (degridding alone, the compiler spreads two polarizations' loads so that
+    // they take longer than in the kernel with both passes: 2.8 against 2.4
+    // ms for supports 8 to 64, 500k visibilities)
+    if (!p.do_grid)
+      return launch_pass<N, DIAG, FORM, W, RING, N == 1 ? 1 : 0>(g, pl, p);
+    if constexpr (FORM != kLinear)
+      if (p.do_degrid && p.has_model)
+        return launch_pass<N, DIAG, FORM, W, RING, 3>(g, pl, p);
+    return launch_pass<N, DIAG, FORM, W, RING, 2>(g, pl, p);
+  } else {
+    return launch_pass<N, DIAG, FORM, W, RING, 0>(g, pl, p);
+  }
 }
 
 // the variants the plan picks from (make_stream_plan)
