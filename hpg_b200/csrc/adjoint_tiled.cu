@@ -331,11 +331,20 @@ __global__ void zero_vals_kernel(double2* v, size_t n) {
 
 }  // namespace
 
+// side of the square region of all rows that shared memory holds
+static int linear_region_side(const hpgb_gridder* g) {
+  const int R =
+      int(std::sqrt(double(kAdjSmemBudget) / (16.0 * g->grid_size[2])));
+  return std::min(R, 128) & ~1;
+}
+
+int linear_tile_side(const hpgb_gridder* g) {
+  return linear_region_side(g) -
+         std::max(g->cf.max_taps_x, g->cf.max_taps_y) + 1;
+}
+
 bool linear_tiled_fits(const hpgb_gridder* g) {
-  const int taps = std::max(g->cf.max_taps_x, g->cf.max_taps_y);
-  int R = int(std::sqrt(double(kAdjSmemBudget) / (16.0 * g->grid_size[2])));
-  R = std::min(R, 128) & ~1;
-  return R - taps + 1 >= 4;
+  return linear_tile_side(g) >= 4;
 }
 
 // Runs op on the tile sort of the batch; *used is false when the region of
@@ -345,10 +354,7 @@ Status linear_op_tiled(hpgb_gridder* g, const void* d_vis, size_t n, int op,
                        const void* in, void* out, bool* used) {
   *used = false;
   const int nrow = int(g->grid_size[2]);
-  const int taps = std::max(g->cf.max_taps_x, g->cf.max_taps_y);
-  int R = int(std::sqrt(double(kAdjSmemBudget) / (16.0 * nrow)));
-  R = std::min(R, 128) & ~1;
-  const int T = R - taps + 1;
+  const int R = linear_region_side(g), T = linear_tile_side(g);
   if (T < 4 || n > size_t(0x7fffffff)) return Status::ok();
   *used = true;
   const int ntx = (int(g->grid_size[0]) + T - 1) / T;

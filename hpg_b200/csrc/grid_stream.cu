@@ -307,6 +307,37 @@ Status grid_stream_device(hpgb_gridder* g, const void* vis, size_t n,
                          used);
 }
 
+// Wide footprints that meet in the same tiles are gathered from, or added
+// into, a tile in shared memory faster than they are in the grid, once a
+// tile's visibilities pay for reading or adding the tile itself.  Nanoseconds
+// on one B200 for c thousand cells (all rows) a visibility and v visibilities
+// a tile: adjoint 4.85 c here against 1.8 + 3 c + 105 / v there, forward
+// 2.3 c against 1.6 + 1.6 c + 95 / v (2 polarizations, supports 8 to 64, 3M
+// visibilities on 2048^2: adjoint 49.3 against 37.2 ms, forward 23.1 against
+// 21.5; 1M on 4096^2: 16.2 against 19.1 and 8.2 against 12.4; 1 polarization,
+// supports 8 to 32, 1M on 1024^2: 2.4 against 3.2 and 1.2 against 2.3).  The
+// tiles' passes (one a tile, of 2048 visibilities at most) must go several
+// times round the SMs.  Slices that go through the ring stay there (4x4
+// planes, supports 8 to 16, 500k visibilities on 1024^2: adjoint 4.0 against
+// 6.9 ms), but for the forward operator on full tiles (3.8 against 3.6 ms with
+// 800 visibilities a tile; 100k on 2048^2, 40 a tile, 0.89 against 0.99).
+static bool tiles_for_linear(const hpgb_gridder* g, const StreamPlan& pl,
+                             size_t n, bool gather) {
+  if (!pl.diag && !(pl.ring && gather)) return false;
+  if (!linear_tiled_fits(g)) return false;
+  const double T = linear_tile_side(g);
+  const double tiles = std::ceil(double(g->grid_size[0]) / T) *
+                       std::ceil(double(g->grid_size[1]) / T);
+  double c = 0.0;
+  for (const CFGroup& G : g->cf.groups) c += double(G.taps_x) * G.taps_y;
+  c *= 1e-3 * double(g->grid_size[2]) / double(g->cf.groups.size());
+  const double v = double(n) / tiles;
+  if (std::max(tiles, double(n) / 2048.0) < 4.0 * 148.0) return false;
+  if (pl.ring) return v > 200.0;
+  return gather ? 2.3 * c > 1.6 + 1.6 * c + 95.0 / v
+                : 4.85 * c > 1.8 + 3.0 * c + 105.0 / v;
+}
+
 Status linear_op_stream(hpgb_gridder* g, const void* d_vis, size_t n, int op,
                         const void* in, void* out, bool* used) {
   *used = false;
@@ -319,7 +350,8 @@ Status linear_op_stream(hpgb_gridder* g, const void* d_vis, size_t n, int op,
   cf.add(g);
   const StreamPlan pl =
       make_stream_plan(g, cf, gather, !gather, gather, set, set, n, false, true);
-  if (!pl.ok) return Status::ok();
+  if (!pl.ok || tiles_for_linear(g, pl, n, gather))
+    return Status::ok();
   *used = true;
   StreamPrep prep;
   HPGB_TRY(prepare_stream(g, d_vis, n,

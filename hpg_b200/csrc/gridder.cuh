@@ -186,6 +186,7 @@ Status linear_op(hpgb_gridder* g, const void* d_vis, size_t n, int op,
 Status linear_op_tiled(hpgb_gridder* g, const void* d_vis, size_t n, int op,
                        const void* in, void* out, bool* used);
 
+int linear_tile_side(const hpgb_gridder* g);
 bool linear_tiled_fits(const hpgb_gridder* g);
 // grid_stream.cu: the same, one visibility per group of warps; *used is false
 // when it cannot take the batch

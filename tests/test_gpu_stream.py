@@ -10,6 +10,8 @@ FP64 in another order (1e-12 of the grid's norm for gridding; predictions are
 rounded once to complex<float>, 4 ulps); the mixed form's FP32 sums are held
 to its 1e-6.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -113,6 +115,64 @@ def test_against_per_visibility_kernels(gpu, case, prec, what):
         np.testing.assert_allclose(a[2], b[2], rtol=1e-12, atol=1e-12)
     else:
         assert not a[1].any()
+
+
+def linear_ops(g, vis, n, npol, shape, kind, seed=3):
+    """D, D^H, G and G^H of one batch, each on the same random input."""
+    import torch
+    gen = torch.Generator(device="cuda:0").manual_seed(seed)
+    dvis = torch.from_numpy(
+        np.frombuffer(vis.tobytes(), np.uint8).copy()).to("cuda:0")
+    crandn = lambda s: torch.randn(s, generator=gen, dtype=torch.complex128,
+                                   device="cuda:0")
+    grid, vals = crandn(shape), crandn((n, npol))
+    g.set_gridding_kernel(kind)
+    lib, out = abi.load(), []
+    for f, a, to_vals in ((lib.hpgb_degrid_linear, grid, True),
+                          (lib.hpgb_degrid_adjoint, vals, False),
+                          (lib.hpgb_grid_linear, vals, False),
+                          (lib.hpgb_grid_adjoint, grid, True)):
+        b = torch.zeros((n, npol) if to_vals else shape,
+                        dtype=torch.complex128, device="cuda:0")
+        torch.cuda.synchronize()
+        abi.check(f(g._h, ctypes.c_void_p(dvis.data_ptr()), n, npol,
+                    ctypes.c_void_p(a.data_ptr()),
+                    ctypes.c_void_p(b.data_ptr())))
+        g.fence()
+        out.append(b.cpu().numpy())
+    return out
+
+
+def assert_linear_ops_agree(g, vis, n, npol, shape):
+    auto = linear_ops(g, vis, n, npol, shape, abi.KERNEL_AUTO)
+    direct = linear_ops(g, vis, n, npol, shape, abi.KERNEL_DIRECT)
+    for a, b in zip(auto, direct):
+        assert rel_norm(a, b) <= 1e-12
+
+
+@pytest.mark.parametrize("case", list(CASES))
+def test_linear_operators(gpu, case):
+    g, vis = make(case, abi.PRECISION_FP64, abi.KERNEL_AUTO)
+    npol, n = CASES[case][0], CASES[case][4]
+    assert_linear_ops_agree(g, vis, n, npol, (2, npol, 150, 131))
+    g.close()
+
+
+@pytest.mark.parametrize("n", [5000, 40000, 160000])
+def test_linear_operators_tile_line(gpu, n):
+    """Batches on both sides of the rule that leaves wide footprints in full
+    tiles to the tile kernels: 27 x 27 tiles of 7, 55 and 220 visibilities
+    (the adjoints' line is near 25, the forward operators' near 130)."""
+    rng = np.random.default_rng(9)
+    gs = (1100, 1111, 2, 1)
+    ext, vals = workloads.separable_cf(
+        (40,), 2, rng.standard_normal(2) + 1j * rng.standard_normal(2), ncube=1)
+    vis = workloads.visibilities(n, 2, gs, (0.05, -0.07), 1.2e9, rng,
+                                 w_frac=0.2, ngroups=1, grad=None, ncube_cf=1)
+    g = Gridder.create(0, 0, n, None, gs, (0.05, -0.07), diag(2), diag(2))
+    g.set_convolution_function(CFArray(2, ext, vals))
+    assert_linear_ops_agree(g, vis, n, 2, (1, 2, 1111, 1100))
+    g.close()
 
 
 def test_wait_limit_and_status(gpu):
