@@ -29,7 +29,8 @@
 // layout, double2 [cube][mrow][y][x]; per-visibility arrays are
 // double2 [n][npol].  The kernels here take one CTA per visibility and
 // accumulate grid outputs with FP64 global atomics; adjoint_tiled.cu runs
-// the same operators on the tile sort of the batch (the default).
+// the same operators on the tile sort of the batch, grid_stream.cu on the
+// stream kernel (the automatic choice of the two: linear_op_stream).
 
 #include "gridder.cuh"
 

@@ -1,8 +1,12 @@
-// grid_batch.cu -- one launch of the tiled kernel over the batches of many
-// gridders (hpgb_grid_visibilities_batch): many independent grids of
+// grid_batch.cu -- one launch over the batches of many gridders
+// (hpgb_grid_visibilities_batch): many independent grids of
 // uneven sizes, each with its own CF set and batch, in one persistent
 // launch, so that the device stays full however small each job is and the
 // whole step is one kernel (and one CUDA graph).
+//
+// Automatic choice: the stream kernel (stream_kernel.cuh) where its plan for
+// the launch says it is the faster one (grid_batch_stream); the tiled kernel
+// otherwise, or when it or its plan was chosen by hand:
 //
 // Every gridder's batch is sorted into uv tiles on its own buffers
 // (tiles.cuh), with the tile side its own CF allows under the launch's

@@ -1,7 +1,8 @@
 // stream_kernel.cuh -- one visibility per group of warps, from its CF slice
 // to the grid, with no uv tiles and no exchange between CTAs: the automatic
-// choice for degridding, gridding and both (grid_stream.cu), for batched
-// launches (grid_batch.cu) and for the linear operators (adjoint_stream.cu).
+// choice for degridding, gridding and both and for the linear operators
+// (grid_stream.cu), and for batched launches (grid_batch.cu), where its plan
+// says it is the faster one.
 //
 // A group of W warps takes one visibility with all its grid rows: it sums
 // the footprint of every row against the model (read from global memory, L2

@@ -85,8 +85,10 @@ enum hpgb_shift_direction { HPGB_SHIFT_FORWARD = 0, HPGB_SHIFT_BACKWARD = 1 };
 enum hpgb_precision { HPGB_PRECISION_FP64 = 0, HPGB_PRECISION_MIXED = 1 };
 
 /* Kernel family used by hpgb_grid_visibilities.
- *  AUTO:   the tiled kernel when the CF fits its shared-memory ring, else
- *          the per-visibility kernels.
+ *  AUTO:   the fastest of the kernels that take the batch: one visibility
+ *          per group of warps, straight into the grid, for all but large
+ *          multi-plane CF slices; for those the tiled kernel when the CF fits
+ *          its shared-memory ring.
  *  DIRECT: per-visibility kernels with global FP64 atomics (the reference's
  *          launch structure; FP64 form only).
  *  TILED:  the tiled kernel, or an error when it cannot take the batch. */
