@@ -4,9 +4,9 @@
 // launch, so that the device stays full however small each job is and the
 // whole step is one kernel (and one CUDA graph).
 //
-// Automatic choice: the stream kernel (stream_kernel.cuh) where its plan for
-// the launch says it is the faster one (grid_batch_stream); the tiled kernel
-// otherwise, or when it or its plan was chosen by hand:
+// Automatic choice: the stream kernel (stream_kernel.cuh) for the gridders
+// whose plans say it is the faster one (grid_batch_stream, one launch); the
+// tiled kernel for the others, or when it or its plan was chosen by hand:
 //
 // Every gridder's batch is sorted into uv tiles on its own buffers
 // (tiles.cuh), with the tile side its own CF allows under the launch's
@@ -234,28 +234,34 @@ Status grid_batch_launch(hpgb_gridder* const* gs, size_t njobs,
 // The batches of many gridders in one launch of the stream kernel, the
 // gridders' blocks of visibilities one after another over its CTAs; their
 // preparation runs on their own streams.
-Status grid_batch_stream(hpgb_gridder* const* gs, size_t njobs,
-                         void* const* d_vis, const size_t* nvis,
-                         unsigned flags, bool* used) {
+static stream::StreamPlan batch_stream_plan(hpgb_gridder* const* gs,
+                                            size_t njobs, const size_t* nvis,
+                                            unsigned flags) {
   using namespace stream;
-  *used = false;
-  hpgb_gridder* g0 = gs[0];
-  const bool mixed = g0->precision == HPGB_PRECISION_MIXED;
-  const bool degrid = flags & HPGB_DO_DEGRID, grid = flags & HPGB_DO_GRID;
-  const bool model = degrid && g0->has_model;
+  const hpgb_gridder* g0 = gs[0];
   CFShape cf;
   size_t total = 0;
   for (size_t j = 0; j < njobs; ++j) {
     cf.add(gs[j]);
     total += nvis[j];
   }
-  if (total == 0 || njobs > size_t(tiled::kMaxBatchJobs)) return Status::ok();
+  if (total == 0 || njobs > size_t(tiled::kMaxBatchJobs)) return StreamPlan();
   const int(*dset[2])[4] = {g0->mt.m, g0->mt.c};
   const int(*gset[2])[4] = {g0->mt.c, g0->mt.m};
-  const StreamPlan pl = make_stream_plan(g0, cf, degrid, grid, g0->has_model,
-                                         dset, gset, total, mixed, true);
-  if (!pl.ok) return Status::ok();
-  *used = true;
+  return make_stream_plan(g0, cf, flags & HPGB_DO_DEGRID, flags & HPGB_DO_GRID,
+                          g0->has_model, dset, gset, total,
+                          g0->precision == HPGB_PRECISION_MIXED, true);
+}
+
+Status grid_batch_stream(hpgb_gridder* const* gs, size_t njobs,
+                         void* const* d_vis, const size_t* nvis,
+                         unsigned flags, const stream::StreamPlan& pl,
+                         unsigned* status) {
+  using namespace stream;
+  hpgb_gridder* g0 = gs[0];
+  const bool mixed = g0->precision == HPGB_PRECISION_MIXED;
+  const bool degrid = flags & HPGB_DO_DEGRID, grid = flags & HPGB_DO_GRID;
+  const bool model = degrid && g0->has_model;
   const cudaStream_t st = g0->stream;
   cudaEvent_t fork = nullptr;
   HPGB_CUDA_TRY(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
@@ -312,7 +318,7 @@ Status grid_batch_stream(hpgb_gridder* const* gs, size_t njobs,
   p.update_weights = (flags & HPGB_UPDATE_GRID_WEIGHTS) != 0;
   p.rec_stride = int(visdata_size(g0->npol));
   p.write_back = 1;
-  p.status = vb.counters.as<unsigned>();
+  p.status = status;
   p.wait_limit_ns = g0->wait_limit_ns;
   return launch_stream(g0, mixed ? stream::kMixed : stream::kFP64, pl, p);
 }
@@ -346,27 +352,55 @@ Status grid_batch_tiled(hpgb_gridder* const* gs, size_t njobs,
     automatic = automatic && gs[j]->kernel_kind == HPGB_KERNEL_AUTO &&
                 gs[j]->tplan.ring_parts == 0 && gs[j]->tplan.chunk_vis == 0 &&
                 gs[j]->tplan.tile_side == 0;
-  if (automatic) {
-    bool used = false;
-    HPGB_TRY(grid_batch_stream(gs, njobs, d_vis, nvis, flags, &used));
-    if (used) return Status::ok();
-  }
   auto taps_class = [](const hpgb_gridder* g) {
     const int t = std::max(g->cf.max_taps_x, g->cf.max_taps_y);
     return t <= 17 ? 0 : t <= 33 ? 1 : t <= 65 ? 2 : 3;
   };
-  std::map<std::pair<int, int>, std::vector<size_t>> groups;
+  std::vector<Plan> own(njobs);
   for (size_t j = 0; j < njobs; ++j) {
-    const Plan own = nvis[j] > 0 ? make_plan(gs[j], flags, mixed, nvis[j], nullptr)
-                                 : Plan();
-    groups[{taps_class(gs[j]), own.ok ? own.R : 0}].push_back(j);
+    if (nvis[j] == 0) continue;
+    own[j] = make_plan(gs[j], flags, mixed, nvis[j], nullptr);
+    // (a batch that the tiled kernel refuses stays refused, and runs nothing)
+    automatic = automatic && own[j].ok;
+  }
+  // the stream kernel takes all gridders, or those that it takes alone (64
+  // jobs of supports 8 to 64 gridded in the mixed form, all through the tiled
+  // kernel before: 2 polarizations 26.8 -> 19.6 ms, 1: 26.8 -> 23.2, 4: 208
+  // -> 196)
+  std::vector<size_t> streamed;
+  stream::StreamPlan splan;
+  if (automatic) {
+    splan = batch_stream_plan(gs, njobs, nvis, flags);
+    std::vector<hpgb_gridder*> sub;
+    std::vector<size_t> sn;
+    for (size_t j = 0; j < njobs; ++j) {
+      if (!splan.ok && !batch_stream_plan(gs + j, 1, nvis + j, flags).ok)
+        continue;
+      streamed.push_back(j);
+      sub.push_back(gs[j]);
+      sn.push_back(nvis[j]);
+    }
+    if (!splan.ok && !sub.empty())
+      splan = batch_stream_plan(sub.data(), sub.size(), sn.data(), flags);
+    if (!splan.ok) streamed.clear();
+  }
+  std::map<std::pair<int, int>, std::vector<size_t>> groups;
+  for (size_t j = 0, k = 0; j < njobs; ++j) {
+    if (k < streamed.size() && streamed[k] == j) {
+      ++k;
+      continue;
+    }
+    groups[{taps_class(gs[j]), own[j].ok ? own[j].R : 0}].push_back(j);
   }
   std::vector<std::vector<size_t>> cls;
   for (auto& kv : groups) cls.push_back(kv.second);
+  if (!streamed.empty()) cls.push_back(streamed);
   const cudaStream_t st = gs[0]->stream;
   unsigned* status = gs[0]->vb.counters.as<unsigned>();
-  const int used = int(cls.size());
-  if (used <= 1) return grid_batch_launch(gs, njobs, d_vis, nvis, flags, status);
+  if (cls.size() <= 1)
+    return streamed.empty()
+               ? grid_batch_launch(gs, njobs, d_vis, nvis, flags, status)
+               : grid_batch_stream(gs, njobs, d_vis, nvis, flags, splan, status);
   cudaEvent_t fork = nullptr;
   HPGB_CUDA_TRY(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
   std::vector<cudaEvent_t> joins;
@@ -389,8 +423,11 @@ Status grid_batch_tiled(hpgb_gridder* const* gs, size_t njobs,
     const cudaStream_t cs = sub[0]->stream;
     if (cs != st) ce = cudaStreamWaitEvent(cs, fork, 0);
     if (ce != cudaSuccess) break;
-    result = grid_batch_launch(sub.data(), sub.size(), sv.data(), sn.data(),
-                               flags, status);
+    result = &c == &cls.back() && !streamed.empty()
+                 ? grid_batch_stream(sub.data(), sub.size(), sv.data(),
+                                     sn.data(), flags, splan, status)
+                 : grid_batch_launch(sub.data(), sub.size(), sv.data(),
+                                     sn.data(), flags, status);
     if (cs != st) {
       cudaEvent_t e = nullptr;
       ce = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);

@@ -178,6 +178,37 @@ def test_batch_wide_supports(gpu, oracle_lib, precision):
         g.close()
 
 
+def test_batch_split_between_kernels(gpu, oracle_lib):
+    """Gridding in the mixed form, where the plan sends the gridders of narrow
+    CFs to the stream kernel and the others to the tiled kernel in one call,
+    plainly and replayed from a graph: the oracle's grids once and twice."""
+    import torch
+    jobs = make_wide_jobs()
+    gs = gridders_for(jobs, abi.PRECISION_MIXED, 0, False)
+    dv = [torch.from_numpy(np.frombuffer(j["vis"].tobytes(), np.uint8).copy()
+                           ).cuda() for j in jobs]
+    hpg_b200.grid_visibilities_batch(gs, dv, on_device=True)
+    gs[0].fence()
+    expected = []
+    for k, (job, g) in enumerate(zip(jobs, gs)):
+        o = oracle_for(oracle_lib, job, False)
+        o.grid_visibilities(job["vis"])
+        expected.append(o)
+        assert g.last_gridding_kernel() == abi.KERNEL_TILED
+        assert rel_norm(g.grid_values(), o.grid) <= 1e-6, k
+        np.testing.assert_allclose(g.grid_weights(), o.weights, rtol=1e-12)
+    with gs[0].capture() as graph:
+        hpg_b200.grid_visibilities_batch(gs, dv, on_device=True)
+    graph.launch()
+    gs[0].fence()
+    for k, (g, o) in enumerate(zip(gs, expected)):
+        assert rel_norm(g.grid_values(), 2 * o.grid) <= 1e-6, k
+        np.testing.assert_allclose(g.grid_weights(), 2 * o.weights, rtol=1e-12)
+    graph.close()
+    for g in gs:
+        g.close()
+
+
 def test_batch_equals_single_calls(gpu):
     """The batched launch against one call per gridder (FP64, degrid+grid):
     residuals bit-identical, grids within 1e-12 (atomic order)."""
