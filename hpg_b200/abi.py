@@ -143,6 +143,8 @@ SIGNATURES = {
     "hpgb_grid_visibilities_batch": ([_P, ctypes.c_size_t, _P, _P, ctypes.c_uint,
                                       ctypes.c_uint, _I, _P], _I),
     "hpgb_debug_withhold_copy": ([_P, ctypes.c_longlong], _I),
+    "hpgb_debug_stream_plan": ([_U, _U, _P, _P, _S, _S, _U, _I, _I, _I, _P],
+                               _I),
     "hpgb_get_tiled_plan": ([_P, ctypes.c_void_p], _I),
     "hpgb_autotune_tiled": ([_P, _P, _S, _U, _U, _I, ctypes.POINTER(_I),
                              ctypes.POINTER(_I)], _I),
@@ -155,6 +157,13 @@ SIGNATURES = {
                                 ctypes.POINTER(ctypes.c_uint64)], _I),
     "hpgb_debug_coords": ([_P, _P, _S, _U, _P], _I),
 }
+
+
+class StreamPlan(ctypes.Structure):
+    """hpgb_stream_plan (include/hpgb.h)."""
+    _fields_ = [(f, ctypes.c_int) for f in
+                ("accepted", "ring", "warps", "smem_bytes", "ring_bytes",
+                 "ring_offset", "slice_bytes")]
 
 
 class TiledPlan(ctypes.Structure):

@@ -950,6 +950,22 @@ int hpgb_debug_withhold_copy(hpgb_gridder* g, long long visibility) {
   });
 }
 
+int hpgb_debug_stream_plan(unsigned npol, unsigned nrow, const int* mueller,
+                           const int* taps, size_t ngroups, size_t nvis,
+                           unsigned flags, int has_model, int precision,
+                           int tiled_takes, hpgb_stream_plan* plan) {
+  return guarded([&]() -> Status {
+    if (!mueller || !taps || !plan)
+      return Status::err(HPGB_ERROR_OTHER, "null argument");
+    if (npol < 1 || npol > 4 || nrow < 1 || nrow > 4)
+      return Status::err(HPGB_ERROR_OTHER,
+                         "polarizations and rows must be 1..4");
+    return stream::debug_stream_plan(
+        npol, nrow, mueller, taps, ngroups, nvis, flags, has_model != 0,
+        precision == HPGB_PRECISION_MIXED, tiled_takes != 0, plan);
+  });
+}
+
 int hpgb_last_gridding_kernel(const hpgb_gridder* g, int* kind) {
   return guarded([&]() -> Status {
     if (!g || !kind) return Status::err(HPGB_ERROR_OTHER, "null argument");

@@ -149,8 +149,10 @@ StreamPlan make_stream_plan(const hpgb_gridder* g, const CFShape& cf,
     // visibilities take 0.63 ms there, 0.49 here.
     pl.ring = mean >= 10 * 1024;
     pl.warps = !pl.ring ? 1 : part > 40 * 1024 ? 7 : 2;
-    if (pl.ring && !(runs_fit && np > 0 &&
-                     layout(pl.warps, true) + part <= kBudget - 1024)) {
+    // whole KB of what the fixed parts leave; the largest slice must fit it
+    if (pl.ring)
+      p.ring_bytes = (kBudget - 1024 - layout(pl.warps, true)) / 1024 * 1024;
+    if (pl.ring && !(runs_fit && np > 0 && part <= p.ring_bytes)) {
       // Slices beyond the ring and the tiled kernel (4x4 planes of supports
       // beyond 45) go to groups of 16 warps, one visibility per SM, whose
       // slices, read again for gridding, stay in L2 (supports 48 and 64, 20k
@@ -165,10 +167,9 @@ StreamPlan make_stream_plan(const hpgb_gridder* g, const CFShape& cf,
     }
   }
   if (pl.ring) {
-    layout(pl.warps, true);
-    p.ring_bytes = (kBudget - 1024 - p.off_ring) / 1024 * 1024;
     pl.smem = p.off_ring + p.ring_bytes;
   } else {
+    p.ring_bytes = 0;
     pl.smem = std::max(layout(pl.warps, false), 1024);
     if (pl.smem * ctas_per_sm(false, n, pl.warps) > kBudget) return pl;
   }
@@ -202,6 +203,37 @@ StreamPlan make_stream_plan(const hpgb_gridder* g, const CFShape& cf,
       1, (nvis + pl.ctas * rounds - 1) / (pl.ctas * rounds)));
   pl.ok = true;
   return pl;
+}
+
+// For tests (no device needed): the plan of a single launch of one gridder.
+Status debug_stream_plan(unsigned npol, unsigned nrow, const int* mueller,
+                         const int* taps, size_t ngroups, size_t nvis,
+                         unsigned flags, bool has_model, bool mixed,
+                         bool tiled_takes, hpgb_stream_plan* out) {
+  hpgb_gridder g;
+  g.npol = npol;
+  g.grid_size[2] = nrow;
+  g.grid_size[3] = 1;
+  int set[4][4];
+  for (int r = 0; r < 4; ++r)
+    for (int c = 0; c < 4; ++c)
+      set[r][c] = r < int(nrow) && c < int(npol) ? mueller[r * npol + c] : -1;
+  for (size_t k = 0; k < ngroups; ++k) {
+    CFGroup G{};
+    G.taps_x = taps[2 * k];
+    G.taps_y = taps[2 * k + 1];
+    G.plane_stride = (G.taps_x * G.taps_y + 1) & ~1;
+    g.cf.groups.push_back(G);
+  }
+  CFShape cf;
+  cf.add(&g);
+  const int(*both[2])[4] = {set, set};
+  const StreamPlan pl = make_stream_plan(
+      &g, cf, flags & HPGB_DO_DEGRID, flags & HPGB_DO_GRID, has_model, both,
+      both, nvis, mixed, tiled_takes);
+  *out = hpgb_stream_plan{pl.ok, pl.ring, pl.warps, pl.smem, pl.p.ring_bytes,
+                          pl.p.off_ring, pl.p.nplanes * cf.max_plane_bytes};
+  return Status::ok();
 }
 
 Status launch_stream(hpgb_gridder* g, int form, const StreamPlan& pl,

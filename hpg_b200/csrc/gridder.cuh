@@ -149,6 +149,13 @@ Status grid_stream(hpgb_gridder* g, void* d_vis, size_t n, unsigned flags,
 Status grid_stream_device(hpgb_gridder* g, const void* vis, size_t n,
                           unsigned flags, void* returned, bool* used);
 
+namespace stream {
+Status debug_stream_plan(unsigned npol, unsigned nrow, const int* mueller,
+                         const int* taps, size_t ngroups, size_t nvis,
+                         unsigned flags, bool has_model, bool mixed,
+                         bool tiled_takes, hpgb_stream_plan* out);
+}
+
 // grid_tiled.cu: the uv tile side of the plan the tiled kernel would take
 // for the batch (false when no plan fits)
 bool tiled_plan_side(const hpgb_gridder* g, unsigned flags, size_t n,

@@ -440,6 +440,27 @@ HPGB_API int hpgb_set_wait_limit(hpgb_gridder* gridder, double seconds);
 HPGB_API int hpgb_debug_withhold_copy(hpgb_gridder* gridder,
                                       long long visibility);
 
+/* Test hook, no counterpart in the reference and no device needed: the plan
+ * of the automatic choice's own kernel (one visibility per group of warps)
+ * for num_visibilities visibilities with the Mueller table
+ * mueller_indexes[num_rows][num_polarizations] (for both signs of w) and CF
+ * groups of taps[num_groups][2] footprint cells.  tiled_takes: whether the
+ * tiled kernel can take the batch. */
+typedef struct hpgb_stream_plan {
+  int accepted;       /* 0: another kernel takes the batch */
+  int ring;           /* CF slices go through a ring in shared memory */
+  int warps;          /* per visibility */
+  int smem_bytes;     /* dynamic shared memory of a CTA */
+  int ring_bytes;     /* of them, the ring's ... */
+  int ring_offset;    /* ... from this byte on */
+  int slice_bytes;    /* largest slice, planes in use */
+} hpgb_stream_plan;
+HPGB_API int hpgb_debug_stream_plan(
+    unsigned num_polarizations, unsigned num_rows, const int* mueller_indexes,
+    const int* taps, size_t num_groups, size_t num_visibilities,
+    unsigned flags, int has_model, int precision, int tiled_takes,
+    hpgb_stream_plan* plan);
+
 /* Which kernel gridded/degridded the gridder's last non-empty batch:
  * HPGB_KERNEL_TILED or HPGB_KERNEL_DIRECT (HPGB_KERNEL_AUTO before the first
  * batch).  No counterpart in the reference: it makes the tiled kernel's
