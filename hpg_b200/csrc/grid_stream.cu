@@ -267,10 +267,10 @@ static Status grid_stream_run(hpgb_gridder* g, void* d_vis, size_t n,
   const bool degrid = flags & HPGB_DO_DEGRID, grid = flags & HPGB_DO_GRID;
   if (n == 0 || n > size_t(0x7fffffff) || !(degrid || grid))
     return Status::ok();
-  const bool mixed = g->precision == HPGB_PRECISION_MIXED;
   // (the mixed form degrids odd grid widths in FP64, by the kernels that do
   // not need its FP32 model)
-  if (mixed && degrid && g->has_model && (g->grid_size[0] & 1))
+  if (g->precision == HPGB_PRECISION_MIXED && degrid && g->has_model &&
+      (g->grid_size[0] & 1))
     return Status::ok();
   // pos_w (w = 1): degrid uses conjugate indexes, grid uses indexes
   const int(*dset[2])[4] = {g->mt.m, g->mt.c};
@@ -279,6 +279,11 @@ static Status grid_stream_run(hpgb_gridder* g, void* d_vis, size_t n,
   cf.add(g);
   int side = 0;
   const bool tiled = tiled_plan_side(g, flags, n, &side);
+  // The mixed form's FP32 arithmetic is the tiled kernel's: what that refuses
+  // (footprints and slices too wide for its shared memory) was always computed
+  // in FP64, by the per-visibility kernels (1 polarization, supports 8 and
+  // 100: error against 64 bits 0 there, 1.0e-7 in the mixed form).
+  const bool mixed = g->precision == HPGB_PRECISION_MIXED && tiled;
   const StreamPlan pl =
       make_stream_plan(g, cf, degrid, grid, g->has_model, dset, gset, n, mixed,
                        tiled);

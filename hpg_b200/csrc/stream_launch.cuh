@@ -63,7 +63,9 @@ Status launch_variants(hpgb_gridder* g, const StreamPlan& pl,
     if (pl.warps == 7) return launch_variant<N, false, FORM, 7, true>(g, pl, p);
     if (pl.warps == 2) return launch_variant<N, false, FORM, 2, true>(g, pl, p);
   } else {
-    if (pl.warps == 16) return launch_variant<N, false, FORM, 16, false>(g, pl, p);
+    // (slices that only the per-visibility kernels would take: FP64)
+    if constexpr (FORM == kFP64)
+      if (pl.warps == 16) return launch_variant<N, false, FORM, 16, false>(g, pl, p);
     if (pl.warps == 1) return launch_variant<N, false, FORM, 1, false>(g, pl, p);
   }
   return Status::err(HPGB_ERROR_OTHER, "stream kernel variant missing");

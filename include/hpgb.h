@@ -81,7 +81,8 @@ enum hpgb_shift_direction { HPGB_SHIFT_FORWARD = 0, HPGB_SHIFT_BACKWARD = 1 };
  *         sums, FP64 grid accumulation, FP64 degridding).
  *  MIXED: FP32 products and FP32 shared-memory tiles, merged into the FP64
  *         grid by compensated (two-sum) flushes; coordinates, phases and
- *         weight sums stay FP64. */
+ *         weight sums stay FP64.  A batch that the tiled kernel cannot take
+ *         is computed in the FP64 form. */
 enum hpgb_precision { HPGB_PRECISION_FP64 = 0, HPGB_PRECISION_MIXED = 1 };
 
 /* Kernel family used by hpgb_grid_visibilities.
