@@ -170,11 +170,15 @@ __device__ __forceinline__ double2 screen_at(const double2* tab, int tx, int X,
 // value's imaginary part and the sum's: sgn*(cf * m) with cf' = (cr, sgn*ci)
 // equals the sum taken with (cr, ci) and (mx, sgn*my), imaginary part times
 // sgn.  Mixed form: packed FP32 products, P = sum cf * (mx, mx) and Q = sum
-// cf * (my, my) componentwise; a lane of a one-warp group sums up to 133
-// cells, so every 16 of them go to a second pair of sums (support 64: error
-// against 64 bits 1.7e-7 in one chain, 1.2e-7 in two, 0.95e-7 with the warp's
-// sums in FP64 too, which cost nothing: 2 polarizations, supports 16 to 64,
-// 300k visibilities 1960 -> 1914 us).
+// cf * (my, my) componentwise.  A lane sums up to 127 * 127 / 32 cells of
+// every row, so chains end early, in a second pair of sums: after 16 cells
+// (18 where six are taken at a time) when each row has its own sums (support
+// 64: error against 64 bits 1.7e-7 in one chain, 1.2e-7 in two, 0.95e-7 with
+// the warp's sums in FP64 too, which cost nothing: 2 polarizations, supports
+// 16 to 64, 300k visibilities 1960 -> 1914 us), after 8 products when all
+// rows add into them (4x4 planes, support 36: 64 products 1.04e-7, 8 0.81e-7,
+// the tiled kernel 1.01e-7; supports 8 to 16, 300k visibilities, both passes:
+// 2580 -> 2605 us).
 template <int A, int FORM>
 struct Sums {
   using V = typename std::conditional<FORM == kMixed, float2, double2>::type;
@@ -608,10 +612,14 @@ stream_kernel(const __grid_constant__ StreamParams p) {
             constexpr bool kAll = !DIAG && !RING;
             constexpr int kU = DIAG ? (FORM == kMixed && N == 2 ? 6 : 4) : kAll ? 1 : 2;
             constexpr int kRows = DIAG ? N : 4;
+            // steps of a chain: 16 cells (18 with six at a time), or with
+            // several rows in a sum, 8 products
+            const int most =
+                DIAG ? (16 + kU - 1) / kU : max(1, 8 / (kU * p.nrow));
             int chain = 0;
 #pragma unroll 1
             for (int c0 = gt; c0 < ncell; c0 += kU * kT) {
-              if (chain == (16 + kU - 1) / kU) {
+              if (chain == most) {
                 sum.settle();
                 chain = 0;
               }

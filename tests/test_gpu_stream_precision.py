@@ -71,3 +71,36 @@ def test_fp64_where_the_tiled_kernel_refuses(gpu, case, what):
                 4 * np.spacing(mag.astype(np.float32))).all()
     else:
         assert rel_norm(a[1], b[1]) <= 1e-12
+
+
+# polarizations, table, supports, visibilities
+TAKEN = {
+    "diag-1": (1, diag(1), (31,), 8000),
+    "diag-2": (2, diag(2), (64,), 5000),
+    "diag-2-few": (2, diag(2), (64,), 1500),
+    "diag-4": (4, diag(4), (30,), 5000),
+    "dense-global-2": (2, dense(2), (14,), 8000),
+    "dense-global-4": (4, dense(4), (7,), 8000),
+    "ring-two-warps-2": (2, dense(2), (30,), 8000),
+    "ring-two-warps-3": (3, dense(3), (20,), 6000),
+    "ring-two-warps-4": (4, dense(4), (16,), 8000),
+    "ring-seven-warps-2": (2, dense(2), (60,), 2500),
+    "ring-seven-warps-4": (4, dense(4), (32,), 2500),
+    "ring-seven-warps-4-wide": (4, dense(4), (36,), 2500),
+}
+
+
+@pytest.mark.parametrize("case", list(TAKEN))
+def test_predictions_as_exact_as_the_tiled_kernels(gpu, case):
+    """The mixed form's sums against the FP64 form, in the variants that take
+    batches from the tiled kernel: no further off than its sums are."""
+    npol, mi, supports, n = TAKEN[case]
+    ref, auto, tiled = (
+        results(npol, mi, supports, n, "predict", prec, kind)[0]
+        .astype(np.complex128) for prec, kind in (
+            (abi.PRECISION_FP64, abi.KERNEL_DIRECT),
+            (abi.PRECISION_MIXED, abi.KERNEL_AUTO),
+            (abi.PRECISION_MIXED, abi.KERNEL_TILED)))
+    err = rel_norm(auto, ref), rel_norm(tiled, ref)
+    print("%s: %.3e, tiled kernel %.3e" % ((case,) + err))
+    assert err[0] <= err[1]
