@@ -401,8 +401,7 @@ Status linear_op_tiled(hpgb_gridder* g, const void* d_vis, size_t n, int op,
   HPGB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount,
                                        g->device));
   auto launch = [&](auto kern) -> Status {
-    HPGB_CUDA_TRY(cudaFuncSetAttribute(
-        kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    HPGB_CUDA_TRY(allow_dynamic_smem(kern, kAdjSmemBudget));
     kern<<<unsigned(sms), kAdjThreads, size_t(smem), g->stream>>>(p);
     HPGB_CUDA_TRY(cudaGetLastError());
     ++g->launches;

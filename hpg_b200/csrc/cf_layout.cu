@@ -357,10 +357,7 @@ Status set_cf(hpgb_gridder* g, unsigned os, unsigned ngroups,
       in_runs = run_smem <= 200 * 1024;
     }
     if (in_runs) {
-      if (run_smem > 48 * 1024)
-        HPGB_CUDA_TRY(cudaFuncSetAttribute(
-            cf_runs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-            int(run_smem)));
+      HPGB_CUDA_TRY(allow_dynamic_smem(cf_runs_kernel));
       const dim3 blocks(unsigned(s.nfine * ((s.nfine + r.B - 1) / r.B)),
                         unsigned((r.run + kMaxRun - 1) / kMaxRun));
       cf_runs_kernel<<<blocks, kRunThreads, run_smem, g->stream>>>(r);

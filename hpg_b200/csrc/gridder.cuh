@@ -14,6 +14,17 @@
 
 namespace hpgb {
 
+// Dynamic shared memory that launches of a kernel may ask for.  A property of
+// the kernel in the whole process, so it is the same at every launch: gridders
+// in other threads launch it with other amounts, and one that lowered the
+// limit between another's call and launch would fail that launch.
+// most: the kernel's own budget, or all that a CTA can have.
+template <typename K>
+cudaError_t allow_dynamic_smem(K* kern, int most = 227 * 1024) {
+  return cudaFuncSetAttribute(
+      kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 // device buffer owned by the gridder
 struct DevBuf {
   void* ptr = nullptr;

@@ -12,8 +12,7 @@ template <int N, bool DIAG, int FORM, int W, bool RING, int PASS>
 Status launch_pass(hpgb_gridder* g, const StreamPlan& pl,
                       const StreamParams& p) {
   auto kern = stream_kernel<N, DIAG, FORM, W, RING, PASS>;
-  HPGB_CUDA_TRY(cudaFuncSetAttribute(
-      kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pl.smem));
+  HPGB_CUDA_TRY(allow_dynamic_smem(kern));
   cudaEvent_t ev[2] = {nullptr, nullptr};
   if (g->profile) {
     HPGB_CUDA_TRY(cudaEventCreate(&ev[0]));

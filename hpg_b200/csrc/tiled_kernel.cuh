@@ -1157,8 +1157,7 @@ Status launch_tiled_kernel(hpgb_gridder* g, const TiledParams& p, int smem,
                             : tiled_kernel<N, MIXED, true, false, BATCH>)
                    : (comp ? tiled_kernel<N, MIXED, false, MIXED, BATCH>
                            : tiled_kernel<N, MIXED, false, false, BATCH>);
-  HPGB_CUDA_TRY(cudaFuncSetAttribute(
-      kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  HPGB_CUDA_TRY(allow_dynamic_smem(kern));
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
