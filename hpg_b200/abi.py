@@ -145,6 +145,7 @@ SIGNATURES = {
     "hpgb_debug_withhold_copy": ([_P, ctypes.c_longlong], _I),
     "hpgb_debug_stream_plan": ([_U, _U, _P, _P, _S, _S, _U, _I, _I, _I, _P],
                                _I),
+    "hpgb_debug_records_in_place": ([_I, _P, _S, _P, ctypes.POINTER(_I)], _I),
     "hpgb_get_tiled_plan": ([_P, ctypes.c_void_p], _I),
     "hpgb_autotune_tiled": ([_P, _P, _S, _U, _U, _I, ctypes.POINTER(_I),
                              ctypes.POINTER(_I)], _I),

@@ -966,6 +966,15 @@ int hpgb_debug_stream_plan(unsigned npol, unsigned nrow, const int* mueller,
   });
 }
 
+int hpgb_debug_records_in_place(int device, const void* vis, size_t bytes,
+                                const void* returned, int* in_place) {
+  return guarded([&]() -> Status {
+    if (!vis || !in_place) return Status::err(HPGB_ERROR_OTHER, "null argument");
+    *in_place = records_in_place(device, vis, bytes, returned);
+    return Status::ok();
+  });
+}
+
 int hpgb_last_gridding_kernel(const hpgb_gridder* g, int* kind) {
   return guarded([&]() -> Status {
     if (!g || !kind) return Status::err(HPGB_ERROR_OTHER, "null argument");

@@ -333,12 +333,32 @@ Status grid_stream(hpgb_gridder* g, void* d_vis, size_t n, unsigned flags,
   return grid_stream_run(g, d_vis, n, flags, false, nullptr, used);
 }
 
+// A copy takes records at any address, of any device or of the host, and
+// into a buffer that overlaps them; the kernels want them aligned, in their
+// own device's memory, and results in the same place or another.
+bool records_in_place(int device, const void* vis, size_t bytes,
+                      const void* returned) {
+  auto usable = [device](const void* p) {
+    cudaPointerAttributes a;
+    if (reinterpret_cast<uintptr_t>(p) % 8 != 0) return false;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == device;
+  };
+  if (!usable(vis)) return false;
+  if (!returned || returned == vis) return true;
+  const uintptr_t a = reinterpret_cast<uintptr_t>(vis);
+  const uintptr_t b = reinterpret_cast<uintptr_t>(returned);
+  return (b >= a ? b - a : a - b) >= bytes && usable(returned);
+}
+
 Status grid_stream_device(hpgb_gridder* g, const void* vis, size_t n,
                           unsigned flags, void* returned, bool* used) {
   *used = false;
-  // (a copy takes records at any address, the kernels want them aligned)
-  if (!automatic(g) || reinterpret_cast<uintptr_t>(vis) % 8 != 0 ||
-      (returned && reinterpret_cast<uintptr_t>(returned) % 8 != 0))
+  if (!automatic(g) ||
+      !records_in_place(g->device, vis, n * visdata_size(g->npol), returned))
     return Status::ok();
   return grid_stream_run(g, const_cast<void*>(vis), n, flags, true, returned,
                          used);

@@ -156,7 +156,10 @@ Status grid_tiled(hpgb_gridder* g, void* d_vis, size_t n, unsigned flags,
 Status grid_stream(hpgb_gridder* g, void* d_vis, size_t n, unsigned flags,
                    bool* used);
 // the same on the caller's device records, without the gridder's copy of
-// them; values are written to `returned` (which may be vis), or nowhere
+// them, where records_in_place says so; values are written to `returned`
+// (which may be vis), or nowhere
+bool records_in_place(int device, const void* vis, size_t bytes,
+                      const void* returned);
 Status grid_stream_device(hpgb_gridder* g, const void* vis, size_t n,
                           unsigned flags, void* returned, bool* used);
 

@@ -462,6 +462,15 @@ HPGB_API int hpgb_debug_stream_plan(
     unsigned flags, int has_model, int precision, int tiled_takes,
     hpgb_stream_plan* plan);
 
+/* Test hook, no counterpart in the reference: whether a gridder of `device`
+ * reads `bytes` of device records where they lie and writes its results to
+ * `returned` (null: nowhere) without copies of its own; where not (another
+ * device's or the host's memory, an address that is no multiple of 8, results
+ * that overlap the records in part), it works on a copy. */
+HPGB_API int hpgb_debug_records_in_place(int device, const void* visibilities,
+                                         size_t bytes, const void* returned,
+                                         int* in_place);
+
 /* Which kernel gridded/degridded the gridder's last non-empty batch:
  * HPGB_KERNEL_TILED or HPGB_KERNEL_DIRECT (HPGB_KERNEL_AUTO before the first
  * batch).  No counterpart in the reference: it makes the tiled kernel's
