@@ -351,7 +351,7 @@ Status grid_batch_tiled(hpgb_gridder* const* gs, size_t njobs,
   for (size_t j = 0; j < njobs; ++j)
     automatic = automatic && gs[j]->kernel_kind == HPGB_KERNEL_AUTO &&
                 gs[j]->tplan.ring_parts == 0 && gs[j]->tplan.chunk_vis == 0 &&
-                gs[j]->tplan.tile_side == 0;
+                gs[j]->tplan.tile_side == 0 && gs[j]->withhold_vis < 0;
   auto taps_class = [](const hpgb_gridder* g) {
     const int t = std::max(g->cf.max_taps_x, g->cf.max_taps_y);
     return t <= 17 ? 0 : t <= 33 ? 1 : t <= 65 ? 2 : 3;

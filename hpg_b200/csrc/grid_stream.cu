@@ -287,7 +287,8 @@ static Status grid_stream_run(hpgb_gridder* g, void* d_vis, size_t n,
   const StreamPlan pl =
       make_stream_plan(g, cf, degrid, grid, g->has_model, dset, gset, n, mixed,
                        tiled);
-  if (!pl.ok) return Status::ok();
+  // (the hook that withholds a copy is for kernels that copy)
+  if (!pl.ok || (g->withhold_vis >= 0 && !pl.ring)) return Status::ok();
   *used = true;
   g->last_kernel = tiled ? HPGB_KERNEL_TILED : HPGB_KERNEL_DIRECT;
   if (in_place && returned && returned != d_vis) {
@@ -317,6 +318,7 @@ static Status grid_stream_run(hpgb_gridder* g, void* d_vis, size_t n,
   p.write_back = !in_place || returned;
   p.status = g->vb.counters.as<unsigned>();
   p.wait_limit_ns = g->wait_limit_ns;
+  if (g->withhold_vis >= 0) p.withhold = prep.descs + g->withhold_vis;
   return launch_stream(g, mixed ? kMixed : kFP64, pl, p);
 }
 

@@ -99,6 +99,8 @@ struct StreamParams {
   double2* vals_out;       // D, G^H: [n][npol]
   unsigned* status;
   unsigned long long wait_limit_ns;
+  // test hook (ring): the copies for this descriptor are never issued
+  const TileDesc* withhold;
 };
 
 // shared memory of the ring variant, from its start
@@ -369,6 +371,7 @@ stream_kernel(const __grid_constant__ StreamParams p) {
                    : "=l"(policy));
     auto issue = [&](const TileDesc* desc, const float2* slice, int s, int roff,
                      int pst, uint32_t q) {
+      if (desc == p.withhold) return;
       const uint32_t pbytes = uint32_t(pst) * 8u;
       const uint32_t need = cf_needed ? uint32_t(p.nplanes) * pbytes : 0u;
       ring_off[s] = roff;

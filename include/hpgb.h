@@ -426,7 +426,7 @@ HPGB_API int hpgb_grid_visibilities_batch(
     unsigned num_polarizations, unsigned flags, int vis_on_device,
     void* const* returned);
 
-/* Bound of every device-side wait of the tiled kernel, in seconds (0.5 by
+/* Bound of every device-side wait of the gridding kernels, in seconds (0.5 by
  * default; 1e-4..60), no counterpart in the reference.  A wait that runs out
  * ends the launch early with an error status: the next hpgb_fence returns
  * HPGB_ERROR_OTHER ("a device-side wait gave up"), the batch's results are
@@ -437,7 +437,10 @@ HPGB_API int hpgb_set_wait_limit(hpgb_gridder* gridder, double seconds);
  * the CTA of grid row 0 that takes the visibility at this position of the
  * tile-sorted batch (of the first gridder, in a batched launch) never
  * issues its bulk copies (-1: none), so that the waits for them run out and
- * the kernel takes its timeout path.  For tests of that path only. */
+ * the kernel takes its timeout path.  While it is set, the automatic choice
+ * takes its own kernel only for single calls whose CF slices that copies, and
+ * withholds the copies of the visibility at this position of its order, else
+ * the tiled kernel.  For tests of that path only. */
 HPGB_API int hpgb_debug_withhold_copy(hpgb_gridder* gridder,
                                       long long visibility);
 
