@@ -138,6 +138,7 @@ SIGNATURES = {
     "hpgb_kernel_launches": ([_P, ctypes.POINTER(ctypes.c_uint64)], _I),
     "hpgb_set_tiled_plan": ([_P, _I, _I], _I),
     "hpgb_last_gridding_kernel": ([_P, ctypes.POINTER(ctypes.c_int)], _I),
+    "hpgb_last_kernel_streamed": ([_P, ctypes.POINTER(ctypes.c_int)], _I),
     "hpgb_set_tiled_plan_ex": ([_P, ctypes.c_void_p], _I),
     "hpgb_set_wait_limit": ([_P, ctypes.c_double], _I),
     "hpgb_grid_visibilities_batch": ([_P, ctypes.c_size_t, _P, _P, ctypes.c_uint,

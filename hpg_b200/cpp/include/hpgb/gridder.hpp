@@ -214,8 +214,8 @@ class Gridder {
   // choice of arithmetic and kernels (no counterpart in the reference)
   opt_error_t set_precision(int precision);
   opt_error_t set_gridding_kernel(int kind);
-  // the tiled kernel's plan (hpgb_set_tiled_plan_ex) and the kernel that
-  // took the last batch (hpgb_last_gridding_kernel)
+  // the tiled kernel's plan (hpgb_set_tiled_plan_ex) and the kernel family of
+  // the last batch (hpgb_last_gridding_kernel)
   opt_error_t set_tiled_plan(const hpgb_tiled_plan& plan);
   hpgb_tiled_plan tiled_plan() const;
   int last_gridding_kernel() const;

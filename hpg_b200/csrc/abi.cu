@@ -908,6 +908,8 @@ int hpgb_grid_visibilities_batch(hpgb_gridder* const* gridders, size_t num,
             vis_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
             st));
     }
+    for (size_t j = 0; j < num; ++j)
+      if (nvis[j] > 0) gridders[j]->last_streamed = false;
     HPGB_TRY(grid_batch_tiled(gridders, num, dvis.data(), nvis, flags));
     for (size_t j = 0; j < num; ++j) {
       if (nvis[j] > 0) gridders[j]->last_kernel = HPGB_KERNEL_TILED;
@@ -979,6 +981,14 @@ int hpgb_last_gridding_kernel(const hpgb_gridder* g, int* kind) {
   return guarded([&]() -> Status {
     if (!g || !kind) return Status::err(HPGB_ERROR_OTHER, "null argument");
     *kind = g->last_kernel;
+    return Status::ok();
+  });
+}
+
+int hpgb_last_kernel_streamed(const hpgb_gridder* g, int* streamed) {
+  return guarded([&]() -> Status {
+    if (!g || !streamed) return Status::err(HPGB_ERROR_OTHER, "null argument");
+    *streamed = g->last_streamed;
     return Status::ok();
   });
 }

@@ -271,9 +271,11 @@ Status linear_op(hpgb_gridder* g, const void* d_vis, size_t n, int op,
     if (used) {
       g->last_kernel = linear_tiled_fits(g) ? HPGB_KERNEL_TILED
                                             : HPGB_KERNEL_DIRECT;
+      g->last_streamed = true;
       return Status::ok();
     }
   }
+  g->last_streamed = false;
   if (g->kernel_kind != HPGB_KERNEL_DIRECT) {
     bool used = false;
     HPGB_TRY(linear_op_tiled(g, d_vis, n, op, in, out, &used));

@@ -16,6 +16,7 @@ Status grid_batch(hpgb_gridder* g, const void* d_vis, size_t n,
   bool streamed = false;
   HPGB_TRY(grid_stream(g, const_cast<void*>(d_vis), n, flags, &streamed));
   if (streamed) return Status::ok();
+  if (n > 0) g->last_streamed = false;
   if (g->kernel_kind != HPGB_KERNEL_DIRECT) {
     bool used = false;
     HPGB_TRY(grid_tiled(g, const_cast<void*>(d_vis), n, flags, &used));

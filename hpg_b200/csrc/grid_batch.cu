@@ -287,6 +287,7 @@ Status grid_batch_stream(hpgb_gridder* const* gs, size_t njobs,
                             stream_sorted(g, nvis[j], model), degrid, grid, false,
                             &prep, js));
     if (model && mixed) HPGB_TRY(tiled::ensure_model32(g, js));
+    g->last_streamed = true;
     StreamJob& b = table->jobs[table->njobs++];
     b.descs = prep.descs;
     b.srefs = prep.srefs;

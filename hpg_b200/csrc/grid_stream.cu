@@ -291,6 +291,7 @@ static Status grid_stream_run(hpgb_gridder* g, void* d_vis, size_t n,
   if (!pl.ok || (g->withhold_vis >= 0 && !pl.ring)) return Status::ok();
   *used = true;
   g->last_kernel = tiled ? HPGB_KERNEL_TILED : HPGB_KERNEL_DIRECT;
+  g->last_streamed = true;
   if (in_place && returned && returned != d_vis) {
     HPGB_CUDA_TRY(cudaMemcpyAsync(returned, d_vis, n * visdata_size(g->npol),
                                   cudaMemcpyDeviceToDevice, g->stream));

@@ -103,6 +103,7 @@ struct hpgb_gridder {
   bool model32_valid = false;
   int kernel_kind = HPGB_KERNEL_AUTO;
   int last_kernel = HPGB_KERNEL_AUTO;  // kernel of the last non-empty batch
+  bool last_streamed = false;          // that was the stream kernel
   // tiled-kernel plan overrides (fields 0: chosen by the plan)
   hpgb_tiled_plan tplan = {0, 0, 0, 0};
   // bound of every device-side wait of the tiled kernel, and its test hook

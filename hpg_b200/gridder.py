@@ -410,10 +410,18 @@ class Gridder:
 
     def last_gridding_kernel(self):
         """abi.KERNEL_TILED or abi.KERNEL_DIRECT: the kernel that took the
-        last non-empty batch (abi.KERNEL_AUTO before any)."""
+        last non-empty batch, or that the automatic choice's own kernel stood
+        in for (abi.KERNEL_AUTO before any)."""
         k = ctypes.c_int()
         check(load().hpgb_last_gridding_kernel(self._h, ctypes.byref(k)))
         return k.value
+
+    def last_kernel_streamed(self):
+        """Whether the automatic choice's own kernel (one visibility per group
+        of warps) took the last non-empty batch or linear operator."""
+        k = ctypes.c_int()
+        check(load().hpgb_last_kernel_streamed(self._h, ctypes.byref(k)))
+        return bool(k.value)
 
     def kernel_launches(self):
         """Kernels this gridder has launched so far."""

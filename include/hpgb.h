@@ -368,7 +368,7 @@ HPGB_API int hpgb_kernel_launches(const hpgb_gridder* gridder,
  * parts, or two or three for CF slices too wide for four (supports up to 64
  * with one or two Mueller planes per grid row).  A plan that does not fit
  * makes the tiled kernel unusable for the batch (HPGB_KERNEL_AUTO then uses
- * the direct kernels; hpgb_last_gridding_kernel tells which ran). */
+ * the direct kernels; hpgb_last_gridding_kernel tells so). */
 HPGB_API int hpgb_set_tiled_plan(hpgb_gridder* gridder, int ring_parts,
                                  int chunk_vis);
 
@@ -474,14 +474,21 @@ HPGB_API int hpgb_debug_records_in_place(int device, const void* visibilities,
                                          size_t bytes, const void* returned,
                                          int* in_place);
 
-/* Which kernel gridded/degridded the gridder's last non-empty batch:
- * HPGB_KERNEL_TILED or HPGB_KERNEL_DIRECT (HPGB_KERNEL_AUTO before the first
- * batch).  No counterpart in the reference: it makes the tiled kernel's
- * fallback to the per-visibility kernels visible to the caller.  The
+/* Which kernel family the gridder's last non-empty batch belonged to:
+ * HPGB_KERNEL_TILED where the tiled kernel can take it, HPGB_KERNEL_DIRECT
+ * where only the per-visibility kernels can or they were selected
+ * (HPGB_KERNEL_AUTO before the first batch).  No counterpart in the reference:
+ * it makes a batch beyond the tiled kernel visible to the caller.  The
  * automatic choice's own kernel (one visibility per group of warps) counts as
- * TILED where the tiled kernel could have taken the batch, else as DIRECT. */
+ * the one that it stands in for; hpgb_last_kernel_streamed names it. */
 HPGB_API int hpgb_last_gridding_kernel(const hpgb_gridder* gridder,
                                        int* kind);
+
+/* Whether the gridder's last non-empty batch (or linear operator) was taken
+ * by the automatic choice's own kernel, one visibility per group of warps:
+ * 1 or 0. */
+HPGB_API int hpgb_last_kernel_streamed(const hpgb_gridder* gridder,
+                                       int* streamed);
 
 /* Autotuner of the tiled kernel, no counterpart in the reference: runs the
  * batch (as hpgb_grid_visibilities would with these flags) three times per
