@@ -359,8 +359,9 @@ class Gridder:
 
     def autotune_tiled(self, visibilities, flags=None, on_device=False):
         """Time the tiled kernel's candidate plans on this batch (grid and
-        weights are left unchanged) and keep the fastest; returns
-        (ring_parts, chunk_vis)."""
+        weights are left unchanged), under abi.KERNEL_AUTO the automatic
+        choice's own kernel too, and keep the fastest; returns (ring_parts,
+        chunk_vis), (0, 0) for the automatic choice's own kernel."""
         if flags is None:
             flags = abi.DO_DEGRID | abi.DO_GRID | abi.UPDATE_GRID_WEIGHTS
         ring = ctypes.c_int()

@@ -495,13 +495,15 @@ HPGB_API int hpgb_last_kernel_streamed(const hpgb_gridder* gridder,
  * candidate plan -- CF ring depths 2..8, then uv tile sides 0, 4, 8, 12 and
  * 16 cells below the largest that fits at the fastest depth and at one part
  * less (the ring takes the bytes a smaller side frees), then tile-pass
- * lengths -- ranks the candidates by their median CUDA-event time (a launch that
+ * lengths, and where the gridder's kernel is HPGB_KERNEL_AUTO and its own
+ * kernel takes the batch, that one -- ranks the candidates by their median CUDA-event time (a launch that
  * reported a device wait timeout does not count), restores the grid and
  * weights on every exit path, and keeps the fastest plan for the gridder's
  * later calls (readable with hpgb_get_tiled_plan), returning its ring depth
- * and pass length.  The mixed form's compensation setting is kept.  Results
+ * and pass length (0 and 0: no plan, the automatic choice's own kernel is
+ * the fastest).  The mixed form's compensation setting is kept.  Results
  * are cached in the process per workload (grid shape, polarizations,
- * Mueller tables, CF group shapes, precision, compensation, flags, model,
+ * Mueller tables, CF group shapes, kernel, precision, compensation, flags, model,
  * log2 of the batch size): a later call with the same workload applies the
  * cached plan at once.  Synchronous; costs about sixty runs of the batch
  * the first time: tune on a representative batch once, then grid. */

@@ -155,3 +155,32 @@ def test_tiled_operators_at_wide_supports(gpu, monkeypatch, npol, grad):
     monkeypatch.setattr(abi, "KERNEL_AUTO", abi.KERNEL_TILED)
     test_adjoint.test_wide_support_dot_products(gpu, npol, abi.KERNEL_TILED,
                                                 grad)
+
+
+def test_autotuner_keeps_the_automatic_choice_where_it_is_faster(gpu):
+    """Small footprints: several times faster through the stream kernel, which
+    a tiled plan would switch off; the tuned call is that one.  The same batch
+    under KERNEL_TILED, and a batch that the stream kernel does not take, get
+    a plan."""
+    g, vis = gridder(2, diag(2), (5, 7, 11, 15), 20000)
+    before = (g.grid_values(), g.grid_weights())
+    assert g.autotune_tiled(vis, abi.DO_GRID) == (0, 0)
+    assert g.autotune_tiled(vis, abi.DO_GRID) == (0, 0)  # from the cache
+    assert g.tiled_plan()["ring_parts"] == 0
+    assert g.last_gridding_kernel() == abi.KERNEL_AUTO  # no batch yet
+    assert not g.last_kernel_streamed()
+    assert np.array_equal(g.grid_values(), before[0])
+    assert np.array_equal(g.grid_weights(), before[1])
+    g.grid_visibilities(vis)
+    g.fence()
+    assert g.last_kernel_streamed()
+    g.close()
+    for args in ((2, diag(2), (5, 7, 11, 15), 20000, abi.KERNEL_TILED),
+                 (4, dense(4), (30,), 7000, abi.KERNEL_AUTO)):
+        g, vis = gridder(*args)
+        ring, _ = g.autotune_tiled(vis, abi.DO_GRID)
+        assert 2 <= ring <= 8 and g.tiled_plan()["ring_parts"] == ring
+        g.grid_visibilities(vis)
+        g.fence()
+        assert not g.last_kernel_streamed()
+        g.close()
