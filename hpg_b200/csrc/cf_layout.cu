@@ -328,7 +328,8 @@ Status set_cf(hpgb_gridder* g, unsigned os, unsigned ngroups,
     const size_t out_bytes =
         size_t(s.nslices) * size_t(s.slice_stride) * sizeof(float2);
     // logical order: one pass, unless a row of the footprint's runs is too
-    // wide for shared memory (supports beyond 750)
+    // wide for shared memory (supports beyond 750) or the values of a position
+    // too many for a launch's blocks (two million)
     RunArgs r;
     size_t run_smem = 0;
     bool in_runs = layout == HPGB_CF_LAYOUT_LOGICAL && s.nslices > 0 &&
@@ -354,7 +355,8 @@ Status set_cf(hpgb_gridder* g, unsigned os, unsigned ngroups,
       // up to 40 KB of rows turned at a time
       r.rows = std::max(1, std::min(s.taps_y, 40960 / (nl * s.taps_x * 8)));
       run_smem = size_t(nl) * size_t(r.rows * s.taps_x | 1) * sizeof(float2);
-      in_runs = run_smem <= 200 * 1024;
+      in_runs = run_smem <= 200 * 1024 &&
+                (r.run + kMaxRun - 1) / kMaxRun <= 65535;
     }
     if (in_runs) {
       HPGB_CUDA_TRY(allow_dynamic_smem(cf_runs_kernel));
