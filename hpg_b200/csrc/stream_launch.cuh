@@ -13,8 +13,10 @@ Status launch_pass(hpgb_gridder* g, const StreamPlan& pl,
                       const StreamParams& p) {
   auto kern = stream_kernel<N, DIAG, FORM, W, RING, PASS>;
   HPGB_CUDA_TRY(allow_dynamic_smem(kern));
+  // (gridding launches only, as the tiled kernel's)
+  const bool profile = FORM != kLinear && g->profile;
   cudaEvent_t ev[2] = {nullptr, nullptr};
-  if (g->profile) {
+  if (profile) {
     HPGB_CUDA_TRY(cudaEventCreate(&ev[0]));
     HPGB_CUDA_TRY(cudaEventCreate(&ev[1]));
     HPGB_CUDA_TRY(cudaEventRecord(ev[0], g->stream));
@@ -23,7 +25,7 @@ Status launch_pass(hpgb_gridder* g, const StreamPlan& pl,
          g->stream>>>(p);
   HPGB_CUDA_TRY(cudaGetLastError());
   ++g->launches;
-  if (g->profile) {
+  if (profile) {
     HPGB_CUDA_TRY(cudaEventRecord(ev[1], g->stream));
     g->prof_events.emplace_back(ev[0], ev[1]);
   }

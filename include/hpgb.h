@@ -533,7 +533,8 @@ HPGB_API int hpgb_graph_destroy(hpgb_graph* graph);
 
 /* Benchmark instrumentation, no counterpart in the reference: while
  * enabled, CUDA events are recorded on the gridder's stream around every
- * launch of the tiled gridding kernel.  hpgb_tiled_kernel_time waits for the
+ * launch of the tiled gridding kernel, or of the automatic choice's own kernel
+ * in its place (linear operators not counted).  hpgb_tiled_kernel_time waits for the
  * stream, returns the summed device time (ms) and the number of launches
  * recorded since the last query, and forgets them. */
 HPGB_API int hpgb_profile_tiled_kernel(hpgb_gridder* gridder, int enable);

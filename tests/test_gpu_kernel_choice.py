@@ -184,3 +184,17 @@ def test_autotuner_keeps_the_automatic_choice_where_it_is_faster(gpu):
         g.fence()
         assert not g.last_kernel_streamed()
         g.close()
+
+
+@pytest.mark.parametrize("kind", [abi.KERNEL_AUTO, abi.KERNEL_TILED],
+                         ids=["auto", "tiled"])
+def test_profiled_launches_are_gridding_launches(gpu, kind):
+    g, vis = gridder(2, diag(2), (8, 14), 700, kind)
+    g.profile_tiled_kernel(True)
+    stream.linear_ops(g, vis, len(vis), 2, (1, 2, 160, 160), kind)
+    assert g.tiled_kernel_time()[1] == 0
+    for _ in range(3):
+        g.grid_visibilities(vis)
+    ms, n = g.tiled_kernel_time()
+    assert n == 3 and ms > 0
+    g.close()
