@@ -294,7 +294,7 @@ class Gridder {
 // the error of a status code (nullopt for success)
 opt_error_t error_of(int status);
 
-// The batches of many gridders in one launch of the tiled kernel
+// The batches of many gridders in one call and few launches
 // (hpgb_grid_visibilities_batch; no counterpart in the reference):
 // gridders[j] grids batches[j] as its grid_visibilities /
 // degrid_grid_visibilities would.  The gridders share polarizations, grid

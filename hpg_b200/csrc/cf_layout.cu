@@ -109,7 +109,7 @@ struct RunArgs {
   const float2* in;
   float2* out;
   double2* wsum;
-  int os, nfine, ext_x, ext_y;
+  int os, nfine, ext_y;
   int taps_x, taps_y, nmueller, ncube, plane_stride;
   long long slice_stride;
   int B;       // fine y offsets per run
@@ -340,7 +340,6 @@ Status set_cf(hpgb_gridder* g, unsigned os, unsigned ngroups,
       r.wsum = ws;
       r.os = int(os);
       r.nfine = s.nfine;
-      r.ext_x = int(e[0]);
       r.ext_y = int(e[1]);
       r.taps_x = s.taps_x;
       r.taps_y = s.taps_y;

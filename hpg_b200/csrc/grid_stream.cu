@@ -53,7 +53,6 @@ StreamPlan make_stream_plan(const hpgb_gridder* g, const CFShape& cf,
   if (nrow < 1 || nrow > 4 || g->cf.groups.empty() || cf.max_side > 127)
     return pl;
   p.nrow = nrow;
-  p.ncube = int(g->grid_size[3]);
   p.do_degrid = degrid;
   p.do_grid = grid;
   p.has_model = has_model;
@@ -408,6 +407,7 @@ Status linear_op_stream(hpgb_gridder* g, const void* d_vis, size_t n, int op,
   if (op >= 2) std::swap(set[0], set[1]);
   CFShape cf;
   cf.add(g);
+  // (slices beyond the ring stay with the tiled or per-visibility operators)
   const StreamPlan pl =
       make_stream_plan(g, cf, gather, !gather, gather, set, set, n, false, true);
   if (!pl.ok || tiles_for_linear(g, pl, n, gather))

@@ -29,7 +29,7 @@ struct CFShape {
 // The plan of a launch over nvis visibilities with g's polarizations and
 // Mueller tables.  dset, gset: the degridding and gridding index tables for
 // w <= 0 and w > 0.  tiles_fp32: the tiled kernel would take FP32 tiles;
-// tiled_takes: it (or the tiled operators) can take the batch.  Not ok where
+// tiled_takes: slices beyond the ring are for another kernel.  Not ok where
 // another kernel is the faster one, or the only one.
 StreamPlan make_stream_plan(const hpgb_gridder* g, const CFShape& cf,
                             bool degrid, bool grid, bool has_model,

@@ -6,21 +6,24 @@
 //
 // A group of W warps takes one visibility with all its grid rows: it sums
 // the footprint of every row against the model (read from global memory, L2
-// mostly: the batch is sorted by uv tile), adds the warps' partial sums
-// through shared memory, forms the residual, and adds the footprint's
-// increments to the FP64 grid with global reductions.
+// mostly: the batch is sorted by uv tile where the grid exceeds that), adds
+// the warps' partial sums through shared memory, forms the residual, and adds
+// the footprint's increments to the FP64 grid with global reductions.
 //
-// What bounds it and why this shape.  The CF slice of a visibility (74 KB at
-// the mean footprint of the full-polarization workload) has to cross HBM
-// once: 3230 cycles per visibility and SM.  Grid tiles in shared memory were
-// the earlier answer to the footprint's additions, at the price of four CTAs
-// per visibility that wait for one another's sums (one grid row of tile
-// each) and a chain of hand-offs of which each takes its latency per
-// visibility.  But reductions on B200 are fast where a warp's lanes fall on
-// consecutive 8-byte words: 640-660 G FP64 reductions a second measured into
-// an L2-resident grid (lanes 16 bytes apart, real part then imaginary part:
-// 330 G), 7 ns for the 4624 of such a visibility, under the 11.5 ns its
-// slice takes.  So lanes work in pairs that exchange one component.
+// What bounds it and why this shape.  The tiled kernel takes ~1000 cycles a
+// visibility and CTA whatever the footprint: its roles hand a visibility on
+// through shared memory, the CTAs of a cluster wait for one another's sums,
+// and tiles want passes and flushes.  Large multi-plane slices hide that (74
+// KB at the mean footprint of the full-polarization workload are 3230 cycles
+// of an SM's share of HBM) and stay there; for footprints of 49 to a few
+// thousand cells with a plane per row it is several times what their CF
+// values and additions cost.  The additions can go straight to the grid:
+// reductions on B200 are fast where a warp's lanes fall on consecutive 8-byte
+// words, 640-660 G FP64 reductions a second measured into an L2-resident grid
+// (lanes 16 bytes apart, real part then imaginary part: 330 G).  So lanes
+// work in pairs that exchange one component.  Small footprints are then bound
+// by instruction issue and the latency of their first loads, wide ones by
+// the CF loads in flight (degridding) and the reductions (gridding).
 //
 // RING: slices stream into a byte ring of shared memory (bulk copies issued
 // by two producer warps, as in tiled_kernel.cuh), each used twice, for
@@ -79,7 +82,7 @@ struct StreamParams {
   StreamJob job;           // the gridder of a launch for one
   const StreamJob* jobs;   // batched launches: the job table, else null
   int njobs;
-  int nrow, ncube;
+  int nrow;
   int do_degrid, do_grid, update_weights, has_model;
   int write_back;   // predictions or residuals go into the records
   int rec_stride;

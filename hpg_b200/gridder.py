@@ -399,14 +399,15 @@ class Gridder:
         return ms.value, n.value
 
     def set_wait_limit(self, seconds):
-        """Bound of every device-side wait of the tiled kernel (seconds)."""
+        """Bound of every device-side wait of the gridding kernels
+        (seconds)."""
         check(load().hpgb_set_wait_limit(self._h, float(seconds)))
 
     def debug_withhold_copy(self, visibility):
-        """Test hook: in later tiled launches, the grid-row-0 CTA that takes
-        the visibility at this position of the tile-sorted batch never
-        issues its copies (-1: none), so that the kernel takes its
-        wait-timeout path."""
+        """Test hook: in later launches of the kernels that copy CF slices,
+        the CTA that takes the visibility at this position of the launch's
+        order never issues its copies (-1: none), so that the kernel takes its
+        wait-timeout path (hpgb_debug_withhold_copy)."""
         check(load().hpgb_debug_withhold_copy(self._h, int(visibility)))
 
     def last_gridding_kernel(self):
@@ -482,7 +483,7 @@ class _Capture:
 def grid_visibilities_batch(gridders, visibilities, update_grid_weights=True,
                             do_degrid=False, return_visibilities=False,
                             on_device=False):
-    """The batches of many gridders in one launch of the tiled kernel
+    """The batches of many gridders in one call and few launches
     (hpgb_grid_visibilities_batch): gridders[j] grids visibilities[j] as
     its own grid_visibilities / degrid_grid_visibilities call would.  With
     return_visibilities, returns one Future per gridder (resolved by

@@ -402,8 +402,9 @@ HPGB_API int hpgb_set_tiled_plan_ex(hpgb_gridder* gridder,
 HPGB_API int hpgb_get_tiled_plan(const hpgb_gridder* gridder,
                                  hpgb_tiled_plan* plan);
 
-/* State::grid_visibilities for the batches of many gridders in ONE launch
- * of the tiled kernel, no counterpart in the reference (which launches per
+/* State::grid_visibilities for the batches of many gridders in one launch
+ * of the automatic choice's own kernel, or launches of the tiled kernel by
+ * support class, no counterpart in the reference (which launches per
  * gridder).  Gridder j takes visibilities[j] (num_visibilities[j] records;
  * host or device memory as vis_on_device says), exactly as
  * hpgb_grid_visibilities(gridders[j], ..., flags, ...) would, and with
@@ -411,13 +412,12 @@ HPGB_API int hpgb_get_tiled_plan(const hpgb_gridder* gridder,
  * (valid after hpgb_fence(gridders[0])).  Up to 96 distinct gridders on one
  * device that share the number of polarizations, grid rows, Mueller tables,
  * precision and compensation setting, and -- when degridding -- whether a
- * model is set; grid sizes, CFs and batch sizes may all differ.  Every
- * gridder's batch is sorted into uv tiles with the tile side its own CF
- * allows, and the tile passes of all of them form one work list of one
- * persistent launch.  The work runs on gridders[0]'s stream, ordered after
- * the work already queued on the others' streams and before work queued on
- * them later (outside a stream capture; inside one, the caller orders the
- * other gridders' work).  Errors: those of hpgb_grid_visibilities, checked
+ * model is set; grid sizes, CFs and batch sizes may all differ.  In a tiled
+ * launch every gridder's batch is sorted into uv tiles with the tile side its
+ * own CF allows, and the tile passes of all of them form one work list.  The
+ * work runs on gridders[0]'s stream, ordered after the work already queued on
+ * the others' streams and before work queued on them later (outside a stream
+ * capture; inside one, the caller orders the other gridders' work).  Errors: those of hpgb_grid_visibilities, checked
  * per gridder, and HPGB_ERROR_OTHER when the gridders differ in a shared
  * property or the tiled kernel cannot take their CFs. */
 HPGB_API int hpgb_grid_visibilities_batch(
@@ -503,7 +503,8 @@ HPGB_API int hpgb_last_kernel_streamed(const hpgb_gridder* gridder,
  * and pass length (0 and 0: no plan, the automatic choice's own kernel is
  * the fastest).  The mixed form's compensation setting is kept.  Results
  * are cached in the process per workload (grid shape, polarizations,
- * Mueller tables, CF group shapes, kernel, precision, compensation, flags, model,
+ * Mueller tables, CF group shapes, kernel, precision, compensation, flags,
+ * model,
  * log2 of the batch size): a later call with the same workload applies the
  * cached plan at once.  Synchronous; costs about sixty runs of the batch
  * the first time: tune on a representative batch once, then grid. */
@@ -534,9 +535,9 @@ HPGB_API int hpgb_graph_destroy(hpgb_graph* graph);
 /* Benchmark instrumentation, no counterpart in the reference: while
  * enabled, CUDA events are recorded on the gridder's stream around every
  * launch of the tiled gridding kernel, or of the automatic choice's own kernel
- * in its place (linear operators not counted).  hpgb_tiled_kernel_time waits for the
- * stream, returns the summed device time (ms) and the number of launches
- * recorded since the last query, and forgets them. */
+ * in its place (linear operators not counted).  hpgb_tiled_kernel_time waits
+ * for the stream, returns the summed device time (ms) and the number of
+ * launches recorded since the last query, and forgets them. */
 HPGB_API int hpgb_profile_tiled_kernel(hpgb_gridder* gridder, int enable);
 HPGB_API int hpgb_tiled_kernel_time(hpgb_gridder* gridder, double* total_ms,
                                     uint64_t* count);
